@@ -711,6 +711,17 @@ __device__ __forceinline__ int shadeClass(int type) {
     return type == kMatLambert ? 0 : (type == kMatConductor || type == kMatRoughDielectric) ? 1 : 2;
 }
 
+// A hit of shading class CLS has one of that class's (at most two) material types.  Said to
+// the compiler, the other types' BSDF code drops out of the class's kernel: the kernels'
+// instruction footprint is what they stall on ("no instruction") when it holds every BSDF.
+// CLS -1: any type.
+template <int CLS>
+__device__ __forceinline__ void narrowType(MaterialRecord &m) {
+    if (CLS == 0) m.type = kMatLambert;
+    if (CLS == 1) m.type = m.type == kMatConductor ? kMatConductor : kMatRoughDielectric;
+    if (CLS == 2) m.type = m.type == kMatDielectric ? kMatDielectric : kMatPlastic;
+}
+
 __device__ __forceinline__ float powerHeuristic(float f, float g) { return (f * f) / (f * f + g * g); }
 
 }  // namespace spgpu

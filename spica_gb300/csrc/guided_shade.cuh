@@ -54,13 +54,16 @@ __device__ __forceinline__ float3 triNormal(const TriRecord &tr) {
 // (1 - alpha) * mix everywhere, MIS weights included.  Sampler streams 0-2 of
 // (seed, fi, sample, b); shadow-ray origins carry the film pixel fi in w, as shadeHit's
 // do.  On a continuation, *fcOut and *pdfOut receive f cos and the proposal's pdf of
-// the sampled direction.
-__device__ __forceinline__ void shadeGuidedLambert(const SceneView &S, float3 ps, float3 n, const MaterialRecord &m,
-                                                   int lightOf, float3 d, float3 beta, bool spec, int b,
-                                                   const Mixture &mix, float alpha, uint32_t seed, uint32_t fi,
-                                                   uint32_t sample, ShadeResult &R, float3 *fcOut, float *pdfOut) {
+// the sampled direction.  shadow(which, origin, direction, contribution) receives the shadow
+// rays, as in shadeHitTo.
+template <class Shadow>
+__device__ __forceinline__ void shadeGuidedLambertTo(const SceneView &S, float3 ps, float3 n, const MaterialRecord &m,
+                                                     int lightOf, float3 d, float3 beta, bool spec, int b,
+                                                     const Mixture &mix, float alpha, uint32_t seed, uint32_t fi,
+                                                     uint32_t sample, ShadeOut &R, float3 *fcOut, float *pdfOut,
+                                                     Shadow shadow) {
     R.emit = mk(0, 0, 0);
-    R.cont = R.sh0 = R.sh1 = false;
+    R.cont = false;
     if ((b == 0 || spec) && lightOf >= 0 && dot(n, -d) > 0.0f) R.emit = beta * xyz(S.lights[lightOf].L);
     MixProposal P{&mix, alpha};
     float3 tg, bg;
@@ -125,10 +128,8 @@ __device__ __forceinline__ void shadeGuidedLambert(const SceneView &S, float3 ps
                 const float3 dd = t2 - oo;
                 const float len = length(dd);
                 if (len > 0.0f) {
-                    R.sh0 = true;
-                    R.s0O = make_float4(oo.x, oo.y, oo.z, __int_as_float(static_cast<int>(fi)));
-                    R.s0D = make_float4(dd.x / len, dd.y / len, dd.z / len, len);
-                    R.s0L = make_float4(c.x, c.y, c.z, 0.0f);
+                    shadow(0, make_float4(oo.x, oo.y, oo.z, __int_as_float(static_cast<int>(fi))),
+                           make_float4(dd.x / len, dd.y / len, dd.z / len, len), make_float4(c.x, c.y, c.z, 0.0f));
                 }
             }
         }
@@ -151,10 +152,9 @@ __device__ __forceinline__ void shadeGuidedLambert(const SceneView &S, float3 ps
                 const float w = powerHeuristic(pdf2, lp);
                 const float3 c = scale * f2 * L2 * (w / pdf2);
                 const float3 oo = offsetOrigin(ps, n, wi2);
-                R.sh1 = true;
-                R.s1O = make_float4(oo.x, oo.y, oo.z, __int_as_float(static_cast<int>(fi)));
-                R.s1D = make_float4(wi2.x, wi2.y, wi2.z, isEnv ? kInfT : tl * (1.0f - 1.0e-5f));
-                R.s1L = make_float4(c.x, c.y, c.z, 0.0f);
+                shadow(1, make_float4(oo.x, oo.y, oo.z, __int_as_float(static_cast<int>(fi))),
+                       make_float4(wi2.x, wi2.y, wi2.z, isEnv ? kInfT : tl * (1.0f - 1.0e-5f)),
+                       make_float4(c.x, c.y, c.z, 0.0f));
             }
         }
     }
@@ -180,6 +180,16 @@ __device__ __forceinline__ void shadeGuidedLambert(const SceneView &S, float3 ps
             R.cD = make_float4(wi.x, wi.y, wi.z, kInfT);
         }
     }
+}
+
+// shadeGuidedLambertTo with the shadow rays kept in the result
+__device__ __forceinline__ void shadeGuidedLambert(const SceneView &S, float3 ps, float3 n, const MaterialRecord &m,
+                                                   int lightOf, float3 d, float3 beta, bool spec, int b,
+                                                   const Mixture &mix, float alpha, uint32_t seed, uint32_t fi,
+                                                   uint32_t sample, ShadeResult &R, float3 *fcOut, float *pdfOut) {
+    R.sh0 = R.sh1 = false;
+    shadeGuidedLambertTo(S, ps, n, m, lightOf, d, beta, spec, b, mix, alpha, seed, fi, sample, R, fcOut, pdfOut,
+                         ShadowsInto{R});
 }
 
 }  // namespace spgpu

@@ -117,13 +117,33 @@ __device__ __forceinline__ void spawnCameraRay(const CameraView &cam, int x, int
 
 // What one bounce produces.  Shadow entries: origin (w = film index bits), direction
 // (w = tmax), contribution.  The continuation ray's origin has w = 0.
-struct ShadeResult {
+struct ShadeOut {
     float3 emit;
     bool cont, spec;
     float3 beta;
     float4 cO, cD;
+};
+struct ShadeResult : ShadeOut {
     bool sh0, sh1;
     float4 s0O, s0D, s0L, s1O, s1D, s1L;
+};
+
+// keeps the shadow rays in a ShadeResult
+struct ShadowsInto {
+    ShadeResult &R;
+    __device__ __forceinline__ void operator()(int which, float4 so, float4 sd, float4 sl) const {
+        if (which == 0) {
+            R.sh0 = true;
+            R.s0O = so;
+            R.s0D = sd;
+            R.s0L = sl;
+        } else {
+            R.sh1 = true;
+            R.s1O = so;
+            R.s1D = sd;
+            R.s1L = sl;
+        }
+    }
 };
 
 // Shade the hit h of ray (o, d) for a path with throughput beta at bounce b.
@@ -132,17 +152,22 @@ struct ShadeResult {
 // direct = true is DirectLightingIntegrator's estimator (no continuation is used):
 // light sampling at every material, since its BSDF::f matches any BxDF sharing a type
 // bit with the non-specular set (bsdf.cc:49-60); the path integrator light-samples only
-// materials with a non-specular BxDF (path.cc:77).
-__device__ __forceinline__ void shadeHit(const SceneView &S, const HitRecord &h, float3 o, float3 d, float3 beta,
-                                         bool spec, int b, int maxDepth, uint32_t seed, uint32_t pixelKey,
-                                         uint32_t sample, int filmIdx, ShadeResult &R, bool direct = false) {
+// materials with a non-specular BxDF (path.cc:77).  CLS: the hit's shading class where the
+// kernel knows it (shadeClass), -1 where it does not.
+// shadow(which, origin, direction, contribution) receives each shadow ray as soon as it is
+// known (which 0: light sampling, 1: BSDF sampling), so that a queueing kernel does not hold
+// two of them in registers through the rest of the shading.
+template <int CLS, class Shadow>
+__device__ __forceinline__ void shadeHitTo(const SceneView &S, const HitRecord &h, float3 o, float3 d, float3 beta,
+                                           bool spec, int b, int maxDepth, uint32_t seed, uint32_t pixelKey,
+                                           uint32_t sample, int filmIdx, ShadeOut &R, bool direct, Shadow shadow) {
     R.emit = mk(0, 0, 0);
     R.cont = false;
-    R.sh0 = R.sh1 = false;
     const TriRecord tr = S.tris[h.prim];
     const float3 n = normalize(cross(xyz(tr.v1) - xyz(tr.v0), xyz(tr.v2) - xyz(tr.v0)));
     const int2 sh = __ldg(&S.slotShade[h.prim]);
-    const MaterialRecord m = S.mats[sh.x];
+    MaterialRecord m = S.mats[sh.x];
+    narrowType<CLS>(m);
     const float3 ps = o + d * h.t;
     // emitted radiance at the first hit or after a specular bounce (path.cc:58-66)
     if ((b == 0 || spec) && sh.y >= 0) {
@@ -156,8 +181,7 @@ __device__ __forceinline__ void shadeHit(const SceneView &S, const HitRecord &h,
         const float3 woL = mk(dot(wo, tg), dot(wo, bg), dot(wo, n));
         const Rand4 r0 = rand4(seed, pixelKey, sample,
                                static_cast<uint32_t>(b), 0u);
-        const Rand4 r1 = rand4(seed, pixelKey, sample,
-                               static_cast<uint32_t>(b), 1u);
+        const Rand4 r1 = rand4(seed, pixelKey, sample, static_cast<uint32_t>(b), 1u);
         // the draws the reference takes from its BxDFs' hidden generator
         const bool hidden = m.type == kMatRoughDielectric || m.type == kMatPlastic;
         const Rand4 r3 = hidden ? rand4(seed, pixelKey, sample, static_cast<uint32_t>(b), 3u) : Rand4{0, 0, 0, 0};
@@ -221,10 +245,8 @@ __device__ __forceinline__ void shadeHit(const SceneView &S, const HitRecord &h,
                     const float3 dd = t2 - o;
                     const float len = length(dd);
                     if (len > 0.0f) {
-                        R.sh0 = true;
-                        R.s0O = make_float4(o.x, o.y, o.z, __int_as_float(filmIdx));
-                        R.s0D = make_float4(dd.x / len, dd.y / len, dd.z / len, len);
-                        R.s0L = make_float4(c.x, c.y, c.z, 0.0f);
+                        shadow(0, make_float4(o.x, o.y, o.z, __int_as_float(filmIdx)),
+                               make_float4(dd.x / len, dd.y / len, dd.z / len, len), make_float4(c.x, c.y, c.z, 0.0f));
                     }
                 }
             }
@@ -251,10 +273,9 @@ __device__ __forceinline__ void shadeHit(const SceneView &S, const HitRecord &h,
                     const float w = powerHeuristic(pdf2, lp);
                     const float3 c = scale * f2 * L2 * (w / pdf2);
                     const float3 o = offsetOrigin(ps, n, wi2);
-                    R.sh1 = true;
-                    R.s1O = make_float4(o.x, o.y, o.z, __int_as_float(filmIdx));
-                    R.s1D = make_float4(wi2.x, wi2.y, wi2.z, isEnv ? kInfT : tl * (1.0f - 1.0e-5f));
-                    R.s1L = make_float4(c.x, c.y, c.z, 0.0f);
+                    shadow(1, make_float4(o.x, o.y, o.z, __int_as_float(filmIdx)),
+                           make_float4(wi2.x, wi2.y, wi2.z, isEnv ? kInfT : tl * (1.0f - 1.0e-5f)),
+                           make_float4(c.x, c.y, c.z, 0.0f));
                 }
             }
         }
@@ -282,6 +303,16 @@ __device__ __forceinline__ void shadeHit(const SceneView &S, const HitRecord &h,
     }
     R.beta = beta;
     R.spec = spec;
+}
+
+// shadeHitTo with the shadow rays kept in the result
+template <int CLS = -1>
+__device__ __forceinline__ void shadeHit(const SceneView &S, const HitRecord &h, float3 o, float3 d, float3 beta,
+                                         bool spec, int b, int maxDepth, uint32_t seed, uint32_t pixelKey,
+                                         uint32_t sample, int filmIdx, ShadeResult &R, bool direct = false) {
+    R.sh0 = R.sh1 = false;
+    shadeHitTo<CLS>(S, h, o, d, beta, spec, b, maxDepth, seed, pixelKey, sample, filmIdx, R, direct,
+                    ShadowsInto{R});
 }
 
 }  // namespace spgpu

@@ -47,10 +47,14 @@ constexpr int kShadeBlockS = 128;
 #define SPGPU_TRACE_MIN_BLOCKS 8
 #endif
 constexpr int kTraceMinBlocks = SPGPU_TRACE_MIN_BLOCKS;   // resident traversal blocks per SM (register budget)
-#ifndef SPGPU_SHADE_MIN_BLOCKS
-#define SPGPU_SHADE_MIN_BLOCKS 6
+// resident shading blocks per SM (register budget) by class: Lambert, the other two
+#ifndef SPGPU_SHADE_MIN_BLOCKS_L
+#define SPGPU_SHADE_MIN_BLOCKS_L 8
 #endif
-constexpr int kShadeMinBlocks = SPGPU_SHADE_MIN_BLOCKS;   // resident shading blocks per SM (register budget)
+#ifndef SPGPU_SHADE_MIN_BLOCKS_G
+#define SPGPU_SHADE_MIN_BLOCKS_G 6
+#endif
+constexpr int shadeMinBlocks(int cls) { return cls == 0 ? SPGPU_SHADE_MIN_BLOCKS_L : SPGPU_SHADE_MIN_BLOCKS_G; }
 #ifndef SPGPU_GUIDED_MIN_BLOCKS
 #define SPGPU_GUIDED_MIN_BLOCKS 4
 #endif
@@ -288,10 +292,19 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
     }
 }
 
-// a shaded hit's emission (at film pixel filmIdx), continuation (back into the pool) and
-// shadow rays; whole warps call this.  Batches count the paths that end here.
+// one shadow ray into the shadow queue; the lanes that have one at the same point of the
+// shading append together
+__device__ __forceinline__ void appendShadow(const StreamArgs &p, float4 so, float4 sd, float4 sl) {
+    const int k = warpAppendS(true, &p.ctr[kCtrShadow]);
+    p.shO[k] = so;
+    p.shD[k] = sd;
+    p.shL[k] = sl;
+}
+
+// a shaded hit's emission (at film pixel filmIdx) and continuation (back into the pool);
+// whole warps call this.  Batches count the paths that end here.
 template <bool BATCH = false>
-__device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const ShadeResult &R, bool live, long long filmIdx,
+__device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const ShadeOut &R, bool live, long long filmIdx,
                                                  int pix, int meta, int sample) {
     if (live && !isBlack(R.emit))
         atomicAdd(&filmOf(p)[filmIdx], make_float4(R.emit.x, R.emit.y, R.emit.z, 0.0f));
@@ -301,18 +314,6 @@ __device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const Shad
         p.rO[k] = make_float4(R.cO.x, R.cO.y, R.cO.z, __int_as_float(pix));
         p.rD[k] = make_float4(R.cD.x, R.cD.y, R.cD.z, packMeta((meta & 255) + 1, R.spec, metaRender(meta)));
         p.rB[k] = make_float4(R.beta.x, R.beta.y, R.beta.z, __int_as_float(sample));
-    }
-    const int s0 = warpAppendS(R.sh0, &p.ctr[kCtrShadow]);
-    if (s0 >= 0) {
-        p.shO[s0] = R.s0O;
-        p.shD[s0] = R.s0D;
-        p.shL[s0] = R.s0L;
-    }
-    const int s1 = warpAppendS(R.sh1, &p.ctr[kCtrShadow]);
-    if (s1 >= 0) {
-        p.shO[s1] = R.s1O;
-        p.shD[s1] = R.s1D;
-        p.shL[s1] = R.s1L;
     }
 }
 
@@ -325,16 +326,24 @@ __device__ __forceinline__ HitRecord hitOfRow(float4 h4) {
     return h;
 }
 
+// One class's queue, a row per thread.  Bound by latency (loads of the hit's triangle,
+// material and light) and by instruction fetch, so the kernel holds its class's BSDFs only
+// (narrowType), shadow rays leave the registers as soon as they are known (shadeHitTo), and
+// the Lambert class, which then needs few registers, keeps 8 CTAs of 128 threads per SM
+// (5 / 6 / 7 / 8: 154.3 / 153.1 / 153.1 / 151.6 ms for a batch of 16 box rooms).  Against
+// every BSDF in each class's kernel and both shadow rays held to the end: that batch 185.3
+// -> 151.6 ms, the 1080p mid-scale render (16 samples) 29.2 -> 27.7 ms, the material room
+// at 333 x 217 (24 samples) 1.94 -> 1.81 ms.
 template <int CLS, bool BATCH>
-__global__ void __launch_bounds__(kShadeBlockS, kShadeMinBlocks) k_sshade(StreamArgs p) {
+__global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(StreamArgs p) {
     const int n = p.ctr[kCtrClass0 + CLS];
     const int stride = gridDim.x * blockDim.x;
     const int nIter = (n + stride - 1) / stride;   // uniform trip count keeps warps whole for the ballots
     const int64_t base = static_cast<int64_t>(CLS) * p.cap;
     for (int it = 0; it < nIter; it++) {
         const int j = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
-        ShadeResult R;
-        R.cont = R.sh0 = R.sh1 = false;
+        ShadeOut R;
+        R.cont = false;
         int pix = 0, meta = 0, sample = 0;
         long long filmIdx = 0;
         if (j < n) {
@@ -352,14 +361,18 @@ __global__ void __launch_bounds__(kShadeBlockS, kShadeMinBlocks) k_sshade(Stream
                 S.nLights = M.nArea;
                 const int fi = mirrored(pix, M.W);
                 filmIdx = M.filmOffset + fi;
-                shadeHit(S, hitOfRow(h4), xyz(o4), xyz(d4), xyz(b4), (meta & 256) != 0, meta & 255, M.maxDepth, M.seed,
-                         static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), static_cast<int>(filmIdx), R, false);
-                R.s0L.w = R.s1L.w = __int_as_float(render);   // the shadow rays' tree
+                shadeHitTo<CLS>(S, hitOfRow(h4), xyz(o4), xyz(d4), xyz(b4), (meta & 256) != 0, meta & 255, M.maxDepth,
+                                M.seed, static_cast<uint32_t>(fi), static_cast<uint32_t>(sample),
+                                static_cast<int>(filmIdx), R, false, [&](int, float4 so, float4 sd, float4 sl) {
+                                    sl.w = __int_as_float(render);   // the shadow ray's tree
+                                    appendShadow(p, so, sd, sl);
+                                });
             } else {
                 const int fi = filmIndexS(p, pix);
                 filmIdx = fi;
-                shadeHit(p.sv, hitOfRow(h4), xyz(o4), xyz(d4), xyz(b4), (meta & 256) != 0, meta & 255, p.maxDepth,
-                         p.seed, static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), fi, R, p.direct != 0);
+                shadeHitTo<CLS>(p.sv, hitOfRow(h4), xyz(o4), xyz(d4), xyz(b4), (meta & 256) != 0, meta & 255,
+                                p.maxDepth, p.seed, static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), fi, R,
+                                p.direct != 0, [&](int, float4 so, float4 sd, float4 sl) { appendShadow(p, so, sd, sl); });
             }
         }
         emitShadeResultS<BATCH>(p, R, j < n, filmIdx, pix, meta, sample);
@@ -411,8 +424,9 @@ __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(Stre
             if (ok) mixtureFromRaw(raw, mix.m);
         }
         if (!ok) break;
-        ShadeResult R;
-        R.cont = R.sh0 = R.sh1 = false;
+        ShadeOut R;
+        R.cont = false;
+        auto shadow = [&](int, float4 so, float4 sd, float4 sl) { appendShadow(p, so, sd, sl); };
         const int pix = __float_as_int(o4.w), meta = __float_as_int(d4.w), sample = __float_as_int(b4.w);
         if (live) {
             const int fi = filmIndexS(p, pix);
@@ -420,14 +434,15 @@ __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(Stre
             const bool spec = (meta & 256) != 0;
             if (depth < p.maxDepth && (p.guidedBounces <= 0 || depth < p.guidedBounces)) {
                 const int2 sh = __ldg(&p.sv.slotShade[__float_as_int(h4.y)]);
+                MaterialRecord m = p.sv.mats[sh.x];
+                narrowType<kMatLambert>(m);
                 float3 fc;
                 float pdf;
-                shadeGuidedLambert(p.sv, ps, nn, p.sv.mats[sh.x], sh.y, xyz(d4), xyz(b4), spec, depth, mix.m,
-                                   p.guideAlpha, p.seed, static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), R,
-                                   &fc, &pdf);
+                shadeGuidedLambertTo(p.sv, ps, nn, m, sh.y, xyz(d4), xyz(b4), spec, depth, mix.m, p.guideAlpha, p.seed,
+                                     static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), R, &fc, &pdf, shadow);
             } else {
-                shadeHit(p.sv, hitOfRow(h4), xyz(o4), xyz(d4), xyz(b4), spec, depth, p.maxDepth, p.seed,
-                         static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), fi, R, false);
+                shadeHitTo<kMatLambert>(p.sv, hitOfRow(h4), xyz(o4), xyz(d4), xyz(b4), spec, depth, p.maxDepth, p.seed,
+                                        static_cast<uint32_t>(fi), static_cast<uint32_t>(sample), fi, R, false, shadow);
             }
         }
         emitShadeResultS(p, R, live, live ? filmIndexS(p, pix) : 0, pix, meta, sample);
