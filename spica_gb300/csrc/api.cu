@@ -197,7 +197,7 @@ void freeScene(Ctx &C) {
 }
 
 // --------------------------------------------------------------------------- tracing
-template <bool ANY, bool STATS>
+template <bool ANY, bool STATS, bool SPLIT>
 __global__ void __launch_bounds__(kTraceBlock, 8) k_trace(const float4 *__restrict__ org, const float4 *__restrict__ dir,
                                                        int n, const WideNode *__restrict__ nodes,
                                                        const TriRecord *__restrict__ tris, uint32_t nNodes,
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_trace(const float4 *__restri
         }
         reinterpret_cast<float4 *>(outHit)[i] = make_float4(L.found ? t : 0.0f, __int_as_float(prim), u, v);
     };
-    tracePersistent<ANY, STATS>(nodes, tris, nNodes, nTris, n, ctl + 1, stack + threadIdx.x, kTraceBlock, &nodeCount,
+    tracePersistent<ANY, STATS, SPLIT>(nodes, tris, nNodes, nTris, n, ctl + 1, stack + threadIdx.x, kTraceBlock, &nodeCount,
                                 &triCount, &overflow, fetch, done);
     if (overflow) atomicOr(ctl, 1);
     if (STATS) {
@@ -254,8 +254,29 @@ int numSMs(int device) {
 // persistent grid: every block resident at once (SMs x blocks per SM)
 int residentTraceBlocks(int device) {
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trace<false, false>, kTraceBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_trace<false, false, false>, kTraceBlock, 0);
     return numSMs(device) * (occ > 0 ? occ : 1);
+}
+
+// k_trace over n rays; ctl: its error flag and ray counter, zeroed before on s
+void enqueueTrace(Ctx &C, int any, bool stats, const float4 *org, const float4 *dir, int n, void *out, int *ctl,
+                  cudaStream_t s) {
+    const int grid = std::min((n + kTraceBlock - 1) / kTraceBlock, residentTraceBlocks(C.device));
+    const uint32_t NN = static_cast<uint32_t>(C.bvh.n_nodes), NT = static_cast<uint32_t>(C.bvh.ntri);
+    auto *hits = any ? nullptr : static_cast<spgpu_hit *>(out);
+    auto *flags = any ? static_cast<uint32_t *>(out) : nullptr;
+    auto launch = [&](auto kernel) {
+        kernel<<<grid, kTraceBlock, 0, s>>>(org, dir, n, C.bvh.nodes, C.bvh.tris, NN, NT, hits, flags, ctl,
+                                            stats ? C.traceStats : nullptr);
+    };
+    if (any) {
+        if (stats) launch(k_trace<true, true, false>);
+        else launch(k_trace<true, false, false>);
+    } else {
+        const bool split = NN >= kSplitMinNodes && n >= kSplitMinRays;
+        if (stats) launch(split ? k_trace<false, true, true> : k_trace<false, true, false>);
+        else launch(split ? k_trace<false, false, true> : k_trace<false, false, false>);
+    }
 }
 
 int launchTrace(Ctx &C, int any, const float *org, const float *dir, int64_t n, void *out, cudaStream_t s,
@@ -279,24 +300,9 @@ int launchTrace(Ctx &C, int any, const float *org, const float *dir, int64_t n, 
     }
     cudaError_t e = cudaMemsetAsync(C.traceErr, 0, 2 * sizeof(int), s);
     if (e != cudaSuccess) return cudaFail("cudaMemsetAsync", e);
-    const int64_t blocksNeeded = (n + kTraceBlock - 1) / kTraceBlock;
-    const int grid = static_cast<int>(std::min<int64_t>(blocksNeeded, static_cast<int64_t>(residentTraceBlocks(C.device))));
-    const uint32_t NN = static_cast<uint32_t>(C.bvh.n_nodes), NT = static_cast<uint32_t>(C.bvh.ntri);
     const float4 *o4 = reinterpret_cast<const float4 *>(org);
     const float4 *d4 = reinterpret_cast<const float4 *>(dir);
-    if (any) {
-        if (stats) k_trace<true, true><<<grid, kTraceBlock, 0, s>>>(o4, d4, static_cast<int>(n), C.bvh.nodes, C.bvh.tris, NN, NT, nullptr,
-                                                                    static_cast<uint32_t *>(out), C.traceErr, C.traceStats);
-        else k_trace<true, false><<<grid, kTraceBlock, 0, s>>>(o4, d4, static_cast<int>(n), C.bvh.nodes, C.bvh.tris, NN, NT, nullptr,
-                                                               static_cast<uint32_t *>(out), C.traceErr, C.traceStats);
-    } else {
-        if (stats) k_trace<false, true><<<grid, kTraceBlock, 0, s>>>(o4, d4, static_cast<int>(n), C.bvh.nodes, C.bvh.tris, NN, NT,
-                                                                     static_cast<spgpu_hit *>(out), nullptr, C.traceErr,
-                                                                     C.traceStats);
-        else k_trace<false, false><<<grid, kTraceBlock, 0, s>>>(o4, d4, static_cast<int>(n), C.bvh.nodes, C.bvh.tris, NN, NT,
-                                                                static_cast<spgpu_hit *>(out), nullptr, C.traceErr,
-                                                                C.traceStats);
-    }
+    enqueueTrace(C, any, stats, o4, d4, static_cast<int>(n), out, C.traceErr, s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cudaFail("trace launch", e);
     return 0;
@@ -871,16 +877,7 @@ int spgpu_trace_host_noalloc(spgpu_ctx *h, int any_hit, const float *org_tmin, c
         if (e == cudaSuccess) e = cudaMemcpyAsync(dO, org_tmin, rayBytes, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dD, dir_tmax, rayBytes, cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) return cudaFail("spgpu_trace_host_noalloc", e);
-        const int64_t blocksNeeded = (n + kTraceBlock - 1) / kTraceBlock;
-        const int grid = static_cast<int>(std::min<int64_t>(blocksNeeded, static_cast<int64_t>(residentTraceBlocks(C.device))));
-        const uint32_t NN = static_cast<uint32_t>(C.bvh.n_nodes), NT = static_cast<uint32_t>(C.bvh.ntri);
-        if (any_hit)
-            k_trace<true, false><<<grid, kTraceBlock, 0, s>>>(dO, dD, static_cast<int>(n), C.bvh.nodes, C.bvh.tris, NN, NT,
-                                                              nullptr, reinterpret_cast<uint32_t *>(dOut), ctl, nullptr);
-        else
-            k_trace<false, false><<<grid, kTraceBlock, 0, s>>>(dO, dD, static_cast<int>(n), C.bvh.nodes, C.bvh.tris, NN,
-                                                               NT, reinterpret_cast<spgpu_hit *>(dOut), nullptr, ctl,
-                                                               nullptr);
+        enqueueTrace(C, any_hit, false, dO, dD, static_cast<int>(n), dOut, ctl, s);
         e = cudaGetLastError();
         if (e != cudaSuccess) return cudaFail("spgpu_trace_host_noalloc: launch", e);
         int flag = 0;

@@ -115,6 +115,10 @@ struct TraceLane {
     int hitSlot;
     float hu, hv;
     bool found;
+    // split form (splitOpen): triangles still to be tested, as bits relative to pbase, and
+    // whether a second such group waits on top of the stack
+    uint32_t pbase, pbits;
+    bool pmore;
 };
 
 __device__ __forceinline__ void laneInit(TraceLane &L, float3 o, float3 d, float tmin, float tmax,
@@ -131,6 +135,8 @@ __device__ __forceinline__ void laneInit(TraceLane &L, float3 o, float3 d, float
     L.hitSlot = -1;
     L.hu = L.hv = 0.0f;
     L.found = false;
+    L.pbase = L.pbits = 0u;
+    L.pmore = false;
 }
 
 // Open the next pending child of the current node group (popping a group from the stack
@@ -284,6 +290,66 @@ __device__ __forceinline__ bool laneStep(TraceLane &L, const WideNode *__restric
     return !nodesLeft(L);
 }
 
+// The split form of a traversal step: splitOpen, then splitTest on the lanes that have a
+// pending triangle.  A lane whose node left several triangles does not hold up the warp while
+// it tests them all; it goes on to its next node with them pending, and waits only when that
+// node leaves a second group.  Triangles are tested in the same order as in laneStep, with
+// some more of them and of the nodes visited before a hit shortens the ray, so the result is
+// the same.  The stack needs one entry more than the tree's depth for the second group.
+template <bool STATS>
+__device__ __forceinline__ bool splitOpen(TraceLane &L, const WideNode *__restrict__ nodes,
+                                          uint32_t nNodes, uint2 *__restrict__ stack, int stride, uint2 *spill,
+                                          uint32_t *nodeCount, bool *overflow) {
+    uint32_t tbase, tbits;
+    if (openChild<STATS>(L, nodes, nNodes, stack, stride, spill, nodeCount, &tbase, &tbits, overflow)) return true;
+    if (tbits) {
+        if (!L.pbits) {
+            L.pbase = tbase;
+            L.pbits = tbits;
+        } else {
+            if (L.sp < kStackShared) stack[L.sp * stride] = make_uint2(tbase, tbits);
+            else spill[L.sp - kStackShared] = make_uint2(tbase, tbits);
+            L.sp++;
+            L.pmore = true;
+        }
+    }
+    return false;
+}
+template <bool ANY, bool STATS>
+__device__ __forceinline__ bool splitTest(TraceLane &L, const TriRecord *__restrict__ tris,
+                                          uint32_t nTris, uint2 *__restrict__ stack, int stride, uint2 *spill,
+                                          uint32_t *triCount, bool *overflow) {
+    const uint32_t ti = L.pbase + static_cast<uint32_t>(__ffs(L.pbits) - 1);
+    L.pbits &= L.pbits - 1u;
+    if (ti >= nTris) {
+        *overflow = true;
+        return true;
+    }
+    if (!L.pbits && L.pmore) {
+        L.sp--;
+        const uint2 g = L.sp < kStackShared ? stack[L.sp * stride] : spill[L.sp - kStackShared];
+        L.pbase = g.x;
+        L.pbits = g.y;
+        L.pmore = false;
+    }
+    return testTriangle<ANY, STATS>(L, tris, nTris, ti, triCount, overflow);
+}
+
+// The split form is taken for trees of at least kSplitMinNodes wide nodes and queues of at
+// least kSplitMinRays rays.  A larger tree's rays test few triangles per node (0.35 on the
+// 2M-triangle scene), a few lanes of a warp at a time; a few dozen triangles in a handful of
+// nodes are tested by most lanes at once, and one at a time they only wait.  Below some
+// millions of rays a launch waits for its slowest rays, whose own chain the split form
+// lengthens.  Measured, whole steps / split: spheres of 256, 1024, 4096 and 16k triangles (36
+// nodes and up), 4M closest-hit rays 0.460 / 0.475, 0.487 / 0.472, 0.601 / 0.569, 0.653 /
+// 0.615 ms; 1M triangles, 1k, 300k, 1.2M, 2.5M and 16M rays 0.084 / 0.101, 0.179 / 0.182,
+// 0.375 / 0.382, 0.616 / 0.600, 3.37 / 3.20 ms; the mid-scale render 26.5 / 25.6 ms; the
+// guided room's 2,418 triangles 4.02 / 4.12 ms, the box room's 36 in a batch 148 / 173 ms.
+// Any-hit batches end at their first hit and gain nothing (2.5M on 1M triangles 0.404 /
+// 0.425 ms); shadow rays of a full pool do (the mid-scale render 25.8 / 25.6 ms).
+constexpr uint32_t kSplitMinNodes = 512;
+constexpr int kSplitMinRays = 1 << 21;
+
 template <bool ANY, bool STATS>
 __device__ __forceinline__ bool traceWide(const WideNode *__restrict__ nodes, const TriRecord *__restrict__ tris,
                                           uint32_t nNodes, uint32_t nTris, float3 o, float3 d, float tmin,
@@ -309,7 +375,7 @@ __device__ __forceinline__ bool traceWide(const WideNode *__restrict__ nodes, co
 // (after Aila and Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG
 // 2009).  fetch(i, &o, &d, &tmin, &tmax) loads ray i; done(i, L) consumes its result.
 // All 32 lanes of each warp execute every iteration of the loop (warp-uniform control),
-// so done() may use warp-collective operations.
+// so done() may use warp-collective operations.  SPLIT: steps of laneStepSplit.
 #ifndef SPGPU_REFILL
 #define SPGPU_REFILL 12
 #endif
@@ -326,13 +392,13 @@ constexpr bool kDeferDone = SPGPU_DEFER_DONE != 0;
 #endif
 constexpr int kStepsPerCheck = SPGPU_STEPS_PER_CHECK;
 
-template <bool ANY, bool STATS, class Fetch, class Done>
+template <bool ANY, bool STATS, bool SPLIT, class Fetch, class Done>
 __device__ __forceinline__ void tracePersistent(const WideNode *__restrict__ nodes,
                                                 const TriRecord *__restrict__ tris, uint32_t nNodes,
                                                 uint32_t nTris, int n, int *rayCounter, uint2 *__restrict__ stack,
                                                 int stride, uint32_t *nodeCount, uint32_t *triCount,
                                                 bool *overflow, Fetch fetch, Done done) {
-    uint2 spill[kStackDepth - kStackShared];
+    uint2 spill[kStackDepth - kStackShared + (SPLIT ? 1 : 0)];
     TraceLane L;
     int ray = -1;            // >= 0 in flight (or finished), -1 idle, -2 no work left
     bool finished = false;   // the ray has finished, its result not yet consumed
@@ -379,9 +445,19 @@ __device__ __forceinline__ void tracePersistent(const WideNode *__restrict__ nod
         if (__all_sync(0xffffffffu, ray == -2)) break;
 #pragma unroll 1
         for (int k = 0; k < kStepsPerCheck; k++) {
-            if (ray >= 0 && !finished) {
-                finished = laneStep<ANY, STATS>(L, nodes, tris, nNodes, nTris, stack, stride, spill, nodeCount,
-                                                triCount, overflow);
+            if constexpr (SPLIT) {
+                bool act = ray >= 0 && !finished;
+                const bool more = act && nodesLeft(L);
+                if (more && !L.pmore)
+                    finished = splitOpen<STATS>(L, nodes, nNodes, stack, stride, spill, nodeCount, overflow);
+                act = act && !finished;
+                if (act && L.pbits)
+                    finished = splitTest<ANY, STATS>(L, tris, nTris, stack, stride, spill, triCount, overflow);
+                if (act && !finished) finished = !L.pbits && !nodesLeft(L);
+            } else {
+                if (ray >= 0 && !finished)
+                    finished = laneStep<ANY, STATS>(L, nodes, tris, nNodes, nTris, stack, stride, spill, nodeCount,
+                                                    triCount, overflow);
             }
         }
     }

@@ -222,7 +222,7 @@ __global__ void k_sregen(StreamArgs p) {
     }
 }
 
-template <bool STATS, bool BATCH>
+template <bool STATS, bool BATCH, bool SPLIT>
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(StreamArgs p) {
     __shared__ uint2 stack[kStackShared * kTraceBlock];
     uint32_t nodeCount = 0, triCount = 0;
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
             *t1 = kInfT;
             *root = p.renders[metaRender(__float_as_int(d4.w))].root;
         };
-        tracePersistent<false, STATS>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
+        tracePersistent<false, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
                                       stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch,
                                       done);
     } else {
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
             *t0 = 0.0f;
             *t1 = kInfT;
         };
-        tracePersistent<false, STATS>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
+        tracePersistent<false, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
                                       stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch,
                                       done);
     }
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(Stre
     if (!ok && threadIdx.x == 0) atomicOr(&p.ctr[kCtrErr], 2);
 }
 
-template <bool STATS, bool BATCH>
+template <bool STATS, bool BATCH, bool SPLIT>
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(StreamArgs p) {
     __shared__ uint2 stack[kStackShared * kTraceBlock];
     const int n = p.ctr[kCtrShadow];
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(Stream
             *t1 = d4.w;
             *root = p.renders[__float_as_int(p.shL[i].w)].root;
         };
-        tracePersistent<true, STATS>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchS],
+        tracePersistent<true, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchS],
                                      stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     } else {
         auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1) {
@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(Stream
             *t0 = 0.0f;
             *t1 = d4.w;
         };
-        tracePersistent<true, STATS>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchS],
+        tracePersistent<true, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchS],
                                      stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     }
     if (overflow) atomicOr(&p.ctr[kCtrErr], 1);
@@ -539,7 +539,7 @@ GridsS streamGrids(int device, int cap, bool guided) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     int occT = 0, occS = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occT, k_sextend<false, false>, kTraceBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occT, k_sextend<false, false, true>, kTraceBlock, 0);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, k_sshade<0, false>, kShadeBlockS, 0);
     GridsS g;
     g.trace = sms * std::max(occT, 1);
@@ -562,11 +562,14 @@ void launchIteration(const StreamArgs &a, const GridsS &g, cudaStream_t s, cudaE
     auto done = [&]() {
         if (ev) cudaEventRecord(ev[(*nev)++], s);
     };
+    // batches are of many small trees
+    const bool split = !BATCH && a.sv.nNodes >= kSplitMinNodes && a.cap >= kSplitMinRays;
     mark(kSRegen);
     k_sregen<BATCH><<<g.regen, 256, 0, s>>>(a);
     done();
     mark(kSExtend);
-    k_sextend<STATS, BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
+    if (split) k_sextend<STATS, BATCH, !BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
+    else k_sextend<STATS, BATCH, false><<<g.trace, kTraceBlock, 0, s>>>(a);
     done();
     mark(kSShadeL);
     if (a.packFwd) k_sshade_guided<<<g.guided, kGTile, kGsSmem, s>>>(a);
@@ -579,7 +582,8 @@ void launchIteration(const StreamArgs &a, const GridsS &g, cudaStream_t s, cudaE
     k_sshade<kMatDielectric, BATCH><<<g.shade, kShadeBlockS, 0, s>>>(a);
     done();
     mark(kSShadow);
-    k_sshadow<STATS, BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
+    if (split) k_sshadow<STATS, BATCH, !BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
+    else k_sshadow<STATS, BATCH, false><<<g.trace, kTraceBlock, 0, s>>>(a);
     done();
     mark(kSAdvance);
     k_sadvance<BATCH><<<1, BATCH ? 256 : 32, 0, s>>>(a);

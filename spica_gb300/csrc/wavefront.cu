@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_extend(PassArgs p, int b) {
             if (k >= 0) p.classQ[c * p.cap + k] = i;
         }
     };
-    tracePersistent<false, STATS>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, cnt + 5, stack + threadIdx.x,
+    tracePersistent<false, STATS, false>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, cnt + 5, stack + threadIdx.x,
                                   kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     if (overflow) atomicOr(p.err, 1);
     if (STATS) {
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_shadow(PassArgs p, int b) {
             }
         }
     };
-    tracePersistent<true, STATS>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, cnt + 6, stack + threadIdx.x,
+    tracePersistent<true, STATS, false>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, cnt + 6, stack + threadIdx.x,
                                  kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     if (overflow) atomicOr(p.err, 1);
     if (STATS) {
