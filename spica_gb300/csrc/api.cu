@@ -671,6 +671,8 @@ int spgpu_upload_scene(spgpu_ctx *h, int32_t ntri, const float *verts, const int
             return rc;
         if ((rc = upload(&C.triLight, triLight.data(), triLight.size(), C.stream))) return rc;
         if ((rc = upload(&C.mats, mats.data(), mats.size(), C.stream))) return rc;
+        C.classMask = 0;
+        for (const MaterialRecord &m : mats) C.classMask |= 1 << shadeClass(m.type);
         if (!lights.empty() && (rc = upload(&C.lights, lights.data(), lights.size(), C.stream))) return rc;
         C.ntri = ntri;
         C.nmat = nmat;

@@ -371,11 +371,15 @@ __device__ __forceinline__ bool traceWide(const WideNode *__restrict__ nodes, co
 
 // Persistent driver: a warp keeps up to 32 rays in flight and refills the lanes whose
 // rays have finished, kRefill or more at a time, from a global ray counter (one
-// atomicAdd per refill), so lanes do not idle while the slowest ray of a batch finishes
+// atomicAdd per refill; the grid is one-dimensional), so lanes do not idle while the slowest ray of a batch finishes
 // (after Aila and Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG
 // 2009).  fetch(i, &o, &d, &tmin, &tmax) loads ray i; done(i, L) consumes its result.
 // All 32 lanes of each warp execute every iteration of the loop (warp-uniform control),
-// so done() may use warp-collective operations.  SPLIT: steps of laneStepSplit.
+// so done() may use warp-collective operations.  SPLIT: steps in
+// the split form.  OWN: where a launch with no more rays than lanes takes them from: the counter
+// (kFromCounter), or each warp its own 32 without touching the counter, counted from the first
+// block or, for the second of two queues in one launch, from the last.
+enum : int { kFromCounter = 0, kOwnFromFirst, kOwnFromLast };
 #ifndef SPGPU_REFILL
 #define SPGPU_REFILL 12
 #endif
@@ -392,7 +396,7 @@ constexpr bool kDeferDone = SPGPU_DEFER_DONE != 0;
 #endif
 constexpr int kStepsPerCheck = SPGPU_STEPS_PER_CHECK;
 
-template <bool ANY, bool STATS, bool SPLIT, class Fetch, class Done>
+template <bool ANY, bool STATS, bool SPLIT, int OWN = kFromCounter, class Fetch, class Done>
 __device__ __forceinline__ void tracePersistent(const WideNode *__restrict__ nodes,
                                                 const TriRecord *__restrict__ tris, uint32_t nNodes,
                                                 uint32_t nTris, int n, int *rayCounter, uint2 *__restrict__ stack,
@@ -403,6 +407,8 @@ __device__ __forceinline__ void tracePersistent(const WideNode *__restrict__ nod
     int ray = -1;            // >= 0 in flight (or finished), -1 idle, -2 no work left
     bool finished = false;   // the ray has finished, its result not yet consumed
     const int lane = threadIdx.x & 31;
+    [[maybe_unused]] const int lanes = gridDim.x * blockDim.x;
+    [[maybe_unused]] bool first = true;
     while (true) {
         if (!kDeferDone) {
             done(finished ? ray : -1, L);
@@ -423,8 +429,15 @@ __device__ __forceinline__ void tracePersistent(const WideNode *__restrict__ nod
                 }
             }
             int base = 0;
-            if (lane == __ffs(idle) - 1) base = atomicAdd(rayCounter, __popc(idle));
-            base = __shfl_sync(0xffffffffu, base, __ffs(idle) - 1);
+            if (OWN == kFromCounter || n > lanes) {
+                if (lane == __ffs(idle) - 1) base = atomicAdd(rayCounter, __popc(idle));
+                base = __shfl_sync(0xffffffffu, base, __ffs(idle) - 1);
+            } else if (first) {
+                base = (OWN == kOwnFromFirst ? blockIdx.x : gridDim.x - 1 - blockIdx.x) * blockDim.x + (threadIdx.x & ~31);
+                first = false;
+            } else {
+                base = n;
+            }
             if (ray == -1) {
                 const int r = base + __popc(idle & ((1u << lane) - 1u));
                 if (r < n) {

@@ -707,7 +707,7 @@ __device__ __forceinline__ float3 bsdfSample(const MaterialRecord &m, float3 wo,
 
 // wavefront shading class (sort key of the material-sorted queues): 0 diffuse, 1 glossy,
 // 2 specular-typed
-__device__ __forceinline__ int shadeClass(int type) {
+__host__ __device__ __forceinline__ int shadeClass(int type) {
     return type == kMatLambert ? 0 : (type == kMatConductor || type == kMatRoughDielectric) ? 1 : 2;
 }
 

@@ -94,7 +94,8 @@ struct StreamQueues {
     float4 *rO = nullptr, *rD = nullptr, *rB = nullptr;   // [cap] the pool
     float4 *qO = nullptr, *qD = nullptr, *qB = nullptr, *qH = nullptr;   // [3 * cap] class queues
     float4 *shO = nullptr, *shD = nullptr, *shL = nullptr;               // [2 * cap] shadow queue
-    int *ctr = nullptr;                                    // per-iteration counters
+    int *ctr = nullptr;                                    // per-iteration counters (a set per iteration in one-pass renders)
+    int *ctrHost = nullptr;                                // pinned: the counters read back
     unsigned long long *big = nullptr;                     // paths started, statistics
     int *doneHost = nullptr;                               // pinned: done flags read back per replay
     cudaEvent_t doneEv[kEvents] = {};
@@ -118,6 +119,7 @@ struct Ctx {
     int *triLight = nullptr;
     int nmat = 0;
     MaterialRecord *mats = nullptr;
+    int classMask = 0;   // bit c: the scene has a material of shading class c
     int nArea = 0;
     LightRecord *lights = nullptr;
     bool hasEnv = false;

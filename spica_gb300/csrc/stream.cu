@@ -73,6 +73,7 @@ constexpr int kDoneRing = StreamQueues::kEvents;
 // iterations, [10] error flags
 enum : int { kCtrRays = 0, kCtrCont, kCtrClass0, kCtrShadow = 5, kCtrFetchE, kCtrFetchS, kCtrDone, kCtrIter, kCtrErr };
 constexpr int kNumCtr = 16;
+constexpr int kMaxIters = 66;   // iterations of a one-pass render: depths 0..64, and the counters after the last
 // 64-bit counters: [0] paths started, [1] paths, [2] closest rays, [3] shadow rays,
 // [4..7] visits (extend nodes, triangles, shadow nodes, triangles); then the call's own
 // parameters, written by the host per render so that one captured graph serves every
@@ -89,6 +90,14 @@ __device__ __forceinline__ float packMeta(int depth, bool spec, int render = 0) 
 }
 __device__ __forceinline__ int metaRender(int meta) { return static_cast<int>(static_cast<unsigned>(meta) >> 9); }
 
+// First statement of the kernels that one-pass renders launch back to back as dependent
+// launches: the next kernel may be set up now, this one's work begins once the last kernel's
+// is complete and visible.  (No effect where a kernel is launched without that attribute.)
+__device__ __forceinline__ void awaitLastKernel() {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+}
+
 struct StreamArgs {
     SceneView sv;
     CameraView cam;
@@ -103,7 +112,13 @@ struct StreamArgs {
     float4 *qO, *qD, *qB, *qH;
     float4 *shO, *shD, *shL;   // shadow queue, 2 * cap rows: (origin, film index), (dir, tmax), contribution
     int *ctr;
+    int *cont;         // continuations written
     unsigned long long *big;
+    // one-pass renders (renderOnePass): every path starts in the first iteration, ctr is the
+    // iteration's own set of counters, cont the next one's ray count; shadowCtr: the counters
+    // of the iteration whose shadow rays k_strace traces (null: none)
+    int onePass;
+    int *shadowCtr;
     // guided renders: the network's packed weights and biases (null: plain BSDF
     // sampling), the proposal's BSDF share, the depths that sample it (0: all but the
     // last), and the scene box that normalises the network's position input
@@ -132,7 +147,7 @@ __device__ __forceinline__ int filmIndexS(const StreamArgs &p, int pix) {
 }
 
 // slots refilled this iteration (every kernel of the iteration derives the same number
-// from the counters, which only k_sadvance changes)
+// from the counters, which only k_sadvance changes); not of one-pass renders
 __device__ __forceinline__ long long totalPaths(const StreamArgs &p) { return static_cast<long long>(p.big[kBigTotal]); }
 __device__ __forceinline__ float4 *filmOf(const StreamArgs &p) { return reinterpret_cast<float4 *>(p.big[kBigFilm]); }
 __device__ __forceinline__ int newPaths(const StreamArgs &p) {
@@ -181,8 +196,10 @@ __device__ __forceinline__ int mirrored(int pix, int W) {
 
 template <bool BATCH>
 __global__ void k_sregen(StreamArgs p) {
-    const int have = p.ctr[kCtrRays];
-    const int nNew = newPaths(p);
+    awaitLastKernel();
+    const int have = p.onePass ? 0 : p.ctr[kCtrRays];
+    const int nNew = p.onePass ? static_cast<int>(totalPaths(p)) : newPaths(p);
+    if (p.onePass && blockIdx.x == 0 && threadIdx.x == 0) p.ctr[kCtrRays] = nNew;
     const long long started = static_cast<long long>(p.big[kBigStarted]);
     // one render: the first sample of the call; batches: the lane's first path in the
     // batch's sequence
@@ -222,11 +239,12 @@ __global__ void k_sregen(StreamArgs p) {
     }
 }
 
-template <bool STATS, bool BATCH, bool SPLIT>
-__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(StreamArgs p) {
-    __shared__ uint2 stack[kStackShared * kTraceBlock];
+// closest hit of the pool's rays into the class queues (every thread of the block)
+// (OWN other than kFromCounter: a one-pass render, whose counter holds all its rays)
+template <bool STATS, bool BATCH, bool SPLIT, int OWN = kFromCounter>
+__device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
     uint32_t nodeCount = 0, triCount = 0;
-    const int n = p.ctr[kCtrRays] + newPaths(p);
+    const int n = p.ctr[kCtrRays] + (OWN != kFromCounter ? 0 : newPaths(p));
     float4 *film = filmOf(p);
     bool overflow = false;
     auto done = [&](int i, const TraceLane &L) {
@@ -271,7 +289,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
             *t1 = kInfT;
             *root = p.renders[metaRender(__float_as_int(d4.w))].root;
         };
-        tracePersistent<false, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
+        tracePersistent<false, STATS, SPLIT, OWN>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
                                       stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch,
                                       done);
     } else {
@@ -281,7 +299,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
             *t0 = 0.0f;
             *t1 = kInfT;
         };
-        tracePersistent<false, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
+        tracePersistent<false, STATS, SPLIT, OWN>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchE],
                                       stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch,
                                       done);
     }
@@ -290,6 +308,12 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
         atomicAdd(&p.big[kBigVisit + 0], static_cast<unsigned long long>(nodeCount));
         atomicAdd(&p.big[kBigVisit + 1], static_cast<unsigned long long>(triCount));
     }
+}
+
+template <bool STATS, bool BATCH, bool SPLIT>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(StreamArgs p) {
+    __shared__ uint2 stack[kStackShared * kTraceBlock];
+    extendQueue<STATS, BATCH, SPLIT>(p, stack);
 }
 
 // one shadow ray into the shadow queue; the lanes that have one at the same point of the
@@ -309,7 +333,7 @@ __device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const Shad
     if (live && !isBlack(R.emit))
         atomicAdd(&filmOf(p)[filmIdx], make_float4(R.emit.x, R.emit.y, R.emit.z, 0.0f));
     if constexpr (BATCH) countEnded(p, live && !R.cont, metaRender(meta));
-    const int k = warpAppendS(R.cont && !p.direct, &p.ctr[kCtrCont]);
+    const int k = warpAppendS(R.cont && !p.direct, p.cont);
     if (k >= 0) {
         p.rO[k] = make_float4(R.cO.x, R.cO.y, R.cO.z, __int_as_float(pix));
         p.rD[k] = make_float4(R.cD.x, R.cD.y, R.cD.z, packMeta((meta & 255) + 1, R.spec, metaRender(meta)));
@@ -336,6 +360,7 @@ __device__ __forceinline__ HitRecord hitOfRow(float4 h4) {
 // at 333 x 217 (24 samples) 1.94 -> 1.81 ms.
 template <int CLS, bool BATCH>
 __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(StreamArgs p) {
+    awaitLastKernel();
     const int n = p.ctr[kCtrClass0 + CLS];
     const int stride = gridDim.x * blockDim.x;
     const int nIter = (n + stride - 1) / stride;   // uniform trip count keeps warps whole for the ballots
@@ -387,6 +412,7 @@ __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(St
 // mixes depths, so one launch covers what the pass-by-pass wavefront does in one guided
 // launch per bounce.
 __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(StreamArgs p) {
+    awaitLastKernel();
     const int n = p.ctr[kCtrClass0 + kMatLambert];
     if (static_cast<int>(blockIdx.x) * kGTile >= n) return;   // no tile for this CTA
     extern __shared__ __align__(128) uint8_t sm[];
@@ -451,10 +477,11 @@ __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(Stre
     if (!ok && threadIdx.x == 0) atomicOr(&p.ctr[kCtrErr], 2);
 }
 
-template <bool STATS, bool BATCH, bool SPLIT>
-__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(StreamArgs p) {
-    __shared__ uint2 stack[kStackShared * kTraceBlock];
-    const int n = p.ctr[kCtrShadow];
+// any hit of the shadow rays counted in ctr, unoccluded ones to the film (every thread of the
+// block)
+template <bool STATS, bool BATCH, bool SPLIT, int OWN = kFromCounter>
+__device__ __forceinline__ void shadowQueue(const StreamArgs &p, int *ctr, uint2 *stack) {
+    const int n = ctr[kCtrShadow];
     float4 *film = filmOf(p);
     bool overflow = false;
     uint32_t nodeCount = 0, triCount = 0;
@@ -473,7 +500,7 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(Stream
             *t1 = d4.w;
             *root = p.renders[__float_as_int(p.shL[i].w)].root;
         };
-        tracePersistent<true, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchS],
+        tracePersistent<true, STATS, SPLIT, OWN>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &ctr[kCtrFetchS],
                                      stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     } else {
         auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1) {
@@ -483,14 +510,31 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(Stream
             *t0 = 0.0f;
             *t1 = d4.w;
         };
-        tracePersistent<true, STATS, SPLIT>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &p.ctr[kCtrFetchS],
+        tracePersistent<true, STATS, SPLIT, OWN>(p.sv.nodes, p.sv.tris, p.sv.nNodes, p.sv.nTris, n, &ctr[kCtrFetchS],
                                      stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     }
-    if (overflow) atomicOr(&p.ctr[kCtrErr], 1);
+    if (overflow) atomicOr(&ctr[kCtrErr], 1);
     if (STATS) {
         atomicAdd(&p.big[kBigVisit + 2], static_cast<unsigned long long>(nodeCount));
         atomicAdd(&p.big[kBigVisit + 3], static_cast<unsigned long long>(triCount));
     }
+}
+
+template <bool STATS, bool BATCH, bool SPLIT>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(StreamArgs p) {
+    __shared__ uint2 stack[kStackShared * kTraceBlock];
+    shadowQueue<STATS, BATCH, SPLIT>(p, p.ctr, stack);
+}
+
+// One-pass renders: an iteration's closest hits (EXTEND) and the last iteration's shadow rays,
+// which do not depend on each other, in one launch; a warp that finds no more of the first
+// goes on with the second.
+template <bool EXTEND, bool SPLIT>
+__global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_strace(StreamArgs p) {
+    __shared__ uint2 stack[kStackShared * kTraceBlock];
+    awaitLastKernel();
+    if constexpr (EXTEND) extendQueue<false, false, SPLIT, kOwnFromFirst>(p, stack);
+    if (p.shadowCtr) shadowQueue<false, false, SPLIT, kOwnFromLast>(p, p.shadowCtr, stack);
 }
 
 // one thread: account the iteration, hand the continuations to the next one, reset the
@@ -538,15 +582,60 @@ struct GridsS {
 GridsS streamGrids(int device, int cap, bool guided) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    int occT = 0, occS = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occT, k_sextend<false, false, true>, kTraceBlock, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occS, k_sshade<0, false>, kShadeBlockS, 0);
+    // resident blocks per SM: properties of the compiled kernels
+    static const int occT = [] {
+        int o = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sextend<false, false, true>, kTraceBlock, 0);
+        return o;
+    }();
+    static const int occS = [] {
+        int o = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sshade<0, false>, kShadeBlockS, 0);
+        return o;
+    }();
     GridsS g;
     g.trace = sms * std::max(occT, 1);
     g.shade = sms * std::max(occS, 1);
     g.regen = std::max(1, std::min((cap + 255) / 256, sms * 8));
     g.guided = guided ? guideTileKernelGrid(reinterpret_cast<const void *>(k_sshade_guided), device, kGsSmem) : 0;
     return g;
+}
+
+// a kernel of an iteration; one-pass renders launch it as dependent on the stream's last kernel
+// (awaitLastKernel), so that its set-up overlaps that kernel's end
+template <class K>
+cudaError_t launchStreamKernel(K kernel, int grid, int block, size_t smem, cudaStream_t s, const StreamArgs &a) {
+    cudaLaunchAttribute dependent;
+    dependent.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    dependent.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &dependent;
+    cfg.numAttrs = a.onePass ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+// the shading kernels of the classes in mask; returns how many
+template <bool BATCH>
+int launchShading(const StreamArgs &a, const GridsS &g, cudaStream_t s, int mask) {
+    int n = 0;
+    if (mask & 1) {
+        if (a.packFwd) launchStreamKernel(k_sshade_guided, g.guided, kGTile, kGsSmem, s, a);
+        else launchStreamKernel(k_sshade<0, BATCH>, g.shade, kShadeBlockS, 0, s, a);
+        n++;
+    }
+    if (mask & 2) {
+        launchStreamKernel(k_sshade<1, BATCH>, g.shade, kShadeBlockS, 0, s, a);
+        n++;
+    }
+    if (mask & 4) {
+        launchStreamKernel(k_sshade<2, BATCH>, g.shade, kShadeBlockS, 0, s, a);
+        n++;
+    }
+    return n;
 }
 
 // one iteration on stream s; with ev, every kernel is bracketed by a pair of events
@@ -571,16 +660,11 @@ void launchIteration(const StreamArgs &a, const GridsS &g, cudaStream_t s, cudaE
     if (split) k_sextend<STATS, BATCH, !BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
     else k_sextend<STATS, BATCH, false><<<g.trace, kTraceBlock, 0, s>>>(a);
     done();
-    mark(kSShadeL);
-    if (a.packFwd) k_sshade_guided<<<g.guided, kGTile, kGsSmem, s>>>(a);
-    else k_sshade<kMatLambert, BATCH><<<g.shade, kShadeBlockS, 0, s>>>(a);
-    done();
-    mark(kSShadeC);
-    k_sshade<kMatConductor, BATCH><<<g.shade, kShadeBlockS, 0, s>>>(a);
-    done();
-    mark(kSShadeD);
-    k_sshade<kMatDielectric, BATCH><<<g.shade, kShadeBlockS, 0, s>>>(a);
-    done();
+    for (int c = 0; c < 3; c++) {
+        mark(kSShadeL + c);
+        launchShading<BATCH>(a, g, s, 1 << c);
+        done();
+    }
     mark(kSShadow);
     if (split) k_sshadow<STATS, BATCH, !BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
     else k_sshadow<STATS, BATCH, false><<<g.trace, kTraceBlock, 0, s>>>(a);
@@ -606,8 +690,9 @@ int ensureStreamQueues(StreamQueues &q, int cap) {
     const size_t c = static_cast<size_t>(cap);
     bool ok = alloc(&q.rO, c) && alloc(&q.rD, c) && alloc(&q.rB, c) && alloc(&q.qO, 3 * c) && alloc(&q.qD, 3 * c) &&
               alloc(&q.qB, 3 * c) && alloc(&q.qH, 3 * c) && alloc(&q.shO, 2 * c) && alloc(&q.shD, 2 * c) &&
-              alloc(&q.shL, 2 * c) && alloc(&q.ctr, kNumCtr) && alloc(&q.big, kNumBig);
+              alloc(&q.shL, 2 * c) && alloc(&q.ctr, kNumCtr * kMaxIters) && alloc(&q.big, kNumBig);
     if (ok) ok = cudaMallocHost(reinterpret_cast<void **>(&q.doneHost), sizeof(int) * kDoneRing) == cudaSuccess;
+    if (ok) ok = cudaMallocHost(reinterpret_cast<void **>(&q.ctrHost), sizeof(int) * kNumCtr * kMaxIters) == cudaSuccess;
     if (ok) {
         for (int k = 0; k < kDoneRing && ok; k++) ok = cudaEventCreateWithFlags(&q.doneEv[k], cudaEventDisableTiming) == cudaSuccess;
     }
@@ -662,6 +747,7 @@ int setupStream(Ctx &C, StreamQueues &q, const float *camera, int W, int H, int 
     a.shD = q.shD;
     a.shL = q.shL;
     a.ctr = q.ctr;
+    a.cont = q.ctr + kCtrCont;
     a.big = q.big;
     if (gv) {
         a.packFwd = gv->packFwd;
@@ -827,6 +913,7 @@ StreamArgs batchLaneArgs(const StreamBatch &SB, int k, cudaGraphConditionalHandl
     a.shD = q.shD;
     a.shL = q.shL;
     a.ctr = q.ctr;
+    a.cont = q.ctr + kCtrCont;
     a.big = q.big;
     a.renders = SB.renders;
     a.pathStart = SB.pathStart;
@@ -968,10 +1055,136 @@ void freeStreamQueues(StreamQueues *q) {
     cudaFree(q->ctr);
     cudaFree(q->big);
     if (q->doneHost) cudaFreeHost(q->doneHost);
+    if (q->ctrHost) cudaFreeHost(q->ctrHost);
     for (int k = 0; k < StreamQueues::kEvents; k++)
         if (q->doneEv[k]) cudaEventDestroy(q->doneEv[k]);
     *q = StreamQueues{};
 }
+
+namespace {
+
+// Paths up to which a one-pass render takes a single lane.  Two lanes' kernels overlap, but
+// each has its own launches: one lane / two, 66k paths 0.43 / 0.46 ms, 1.7M paths in the
+// material room 1.37 / 1.32 ms, 1.8M guided 3.31 / 3.32 ms.
+constexpr long long kOneLanePaths = 1 << 18;
+
+// A render whose paths all fit the pools' slots at once.  Every path starts in the first
+// iteration and iteration b handles depth b, so the iterations are known beforehand: no refill,
+// no done flag, no replays past the end, and no graph to capture for a new camera.  Each
+// iteration has its own counters (nothing resets them), its shadow rays are traced in the next
+// iteration's launch, and the classes that the scene has no material of are not launched: two
+// kernels for an iteration of a one-class scene instead of seven.  Bound by the launches' own
+// latency at the small end.  Against the refilling loop's replays: box room, 64 x 64, 16
+// samples (host film) 1.00 -> 0.43 ms; material room, 333 x 217, 24 samples 1.82 -> 1.32;
+// guided room, 640 x 360, 8 samples 4.04 -> 3.32.
+int renderOnePass(Ctx &C, const float *camera, int W, int H, int spp, int sampleOffset, int maxDepth, uint32_t seed,
+                  int integrator, float4 *film, unsigned long long *statsOut, float *msOut, cudaStream_t stream,
+                  const GuideView *gv) {
+    const long long total = static_cast<long long>(W) * H * spp;
+    const int lanes = total <= kOneLanePaths ? 1 : std::max(1, std::min(spp, Ctx::kPoolLanes));
+    StreamArgs a[Ctx::kPoolLanes];
+    StreamInit init[Ctx::kPoolLanes];
+    cudaStream_t ls[Ctx::kPoolLanes];
+    int first = sampleOffset;
+    for (int k = 0; k < lanes; k++) {
+        const int sppK = spp / lanes + (k < spp % lanes ? 1 : 0);
+        if (int rc = setupStream(C, C.sq[k], camera, W, H, sppK, maxDepth, seed, integrator, gv, &a[k])) return rc;
+        a[k].onePass = 1;
+        init[k] = streamInit(static_cast<long long>(W) * H * sppK, first, film);
+        first += sppK;
+        ls[k] = k == 0 ? stream : C.laneStream[k - 1];
+    }
+    // a path's last vertex (depth maxDepth) is shaded in the last iteration and has no shadow
+    // rays; direct lighting has one vertex, whose shadow rays take a launch of their own
+    const bool direct = integrator == SPGPU_INTEGRATOR_DIRECT;
+    const int iters = direct ? 1 : maxDepth + 1;
+    const GridsS g = streamGrids(C.device, a[0].cap, a[0].packFwd != nullptr);
+    const bool split = a[0].sv.nNodes >= kSplitMinNodes && a[0].cap >= kSplitMinRays;
+    long long launches = 0;
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    cudaError_t e = cudaEventRecord(e0, stream);
+    if (e == cudaSuccess && lanes > 1) e = cudaEventRecord(C.laneFork, stream);
+    for (int k = 0; k < lanes && e == cudaSuccess; k++) {
+        if (k > 0) e = cudaStreamWaitEvent(ls[k], C.laneFork, 0);
+        if (e == cudaSuccess) e = cudaMemsetAsync(C.sq[k].ctr, 0, sizeof(int) * kNumCtr * (iters + 1), ls[k]);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(C.sq[k].big, init[k].big, sizeof(init[k].big), cudaMemcpyHostToDevice, ls[k]);
+        if (e != cudaSuccess) break;
+        k_sregen<false><<<g.regen, 256, 0, ls[k]>>>(a[k]);
+        launches++;
+    }
+    constexpr int kLookAhead = 16;   // deep renders: iterations launched between two looks at the paths left
+    int done = iters;                // iterations launched
+    for (int it = 0; it < iters && e == cudaSuccess; it++) {
+        if (it > 0 && it % kLookAhead == 0) {
+            int left = 0;
+            for (int k = 0; k < lanes && e == cudaSuccess; k++) {
+                e = cudaMemcpyAsync(C.sq[k].ctrHost, a[k].cont, sizeof(int), cudaMemcpyDeviceToHost, ls[k]);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(ls[k]);
+                if (e == cudaSuccess) left += C.sq[k].ctrHost[0];
+            }
+            if (e == cudaSuccess && left == 0) {
+                done = it;
+                break;
+            }
+        }
+        for (int k = 0; k < lanes && e == cudaSuccess; k++) {
+            StreamArgs &p = a[k];
+            p.ctr = C.sq[k].ctr + kNumCtr * it;
+            p.cont = p.ctr + kNumCtr + kCtrRays;
+            p.shadowCtr = it > 0 ? p.ctr - kNumCtr : nullptr;
+            if (split) launchStreamKernel(k_strace<true, true>, g.trace, kTraceBlock, 0, ls[k], p);
+            else launchStreamKernel(k_strace<true, false>, g.trace, kTraceBlock, 0, ls[k], p);
+            launches++;
+            launches += launchShading<false>(p, g, ls[k], C.classMask);
+            e = cudaGetLastError();
+        }
+    }
+    if (direct || done < iters) {   // the shadow rays of the last iteration launched
+        for (int k = 0; k < lanes && e == cudaSuccess; k++) {
+            a[k].shadowCtr = C.sq[k].ctr + kNumCtr * (done - 1);
+            if (split) launchStreamKernel(k_strace<false, true>, g.trace, kTraceBlock, 0, ls[k], a[k]);
+            else launchStreamKernel(k_strace<false, false>, g.trace, kTraceBlock, 0, ls[k], a[k]);
+            launches++;
+            e = cudaGetLastError();
+        }
+    }
+    for (int k = 0; k < lanes && e == cudaSuccess; k++)
+        e = cudaMemcpyAsync(C.sq[k].ctrHost, C.sq[k].ctr, sizeof(int) * kNumCtr * (done + 1), cudaMemcpyDeviceToHost, ls[k]);
+    for (int k = 1; k < lanes && e == cudaSuccess; k++) {
+        e = cudaEventRecord(C.laneJoin[k - 1], ls[k]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, C.laneJoin[k - 1], 0);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(e1, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    float ms = 0.0f;
+    if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    if (e != cudaSuccess) return cudaFail("spgpu_render", e);
+    int err = 0;
+    for (int k = 0; k < lanes; k++) {
+        const int *c = C.sq[k].ctrHost;
+        statsOut[0] += init[k].big[kBigTotal];
+        for (int it = 0; it < done; it++, c += kNumCtr) {
+            statsOut[1] += static_cast<unsigned long long>(c[kCtrRays]);
+            statsOut[2] += static_cast<unsigned long long>(c[kCtrShadow]);
+            err |= c[kCtrErr];
+        }
+    }
+    statsOut[3] = static_cast<unsigned long long>(launches);
+    *msOut = ms;
+    if (err) {
+        setError(err & 1 ? "spgpu_render: traversal stack overflow"
+                         : "spgpu_render: tensor-core wait of the guided shading timed out");
+        return SPGPU_EKERNEL;
+    }
+    return 0;
+}
+
+}  // namespace
 
 int renderStream(Ctx *ctx, const float *camera, int W, int H, int spp, int sampleOffset, int maxDepth, uint32_t seed,
                  int integrator, float4 *film, unsigned long long *statsOut, float *msOut, cudaStream_t stream,
@@ -980,6 +1193,11 @@ int renderStream(Ctx *ctx, const float *camera, int W, int H, int spp, int sampl
     for (int j = 0; j < 4; j++) statsOut[j] = 0;
     *msOut = 0.0f;
     if (spp <= 0 || W <= 0 || H <= 0) return 0;
+    // one pass where each lane's samples fit its pool's slots
+    const int perLane = (spp + Ctx::kPoolLanes - 1) / Ctx::kPoolLanes;
+    if (static_cast<long long>(W) * H * perLane <= Ctx::kStreamSlots)
+        return renderOnePass(C, camera, W, H, spp, sampleOffset, maxDepth, seed, integrator, film, statsOut, msOut,
+                             stream, gv);
     // pool lanes: lane k renders a contiguous share of the samples, lane 0 on the caller's
     // stream, lane k > 0 on the context's lane stream k - 1
     const int lanes = std::max(1, std::min(spp, Ctx::kPoolLanes));
