@@ -1,0 +1,71 @@
+"""The film resolve's fast evaluations against the reference's arithmetic in FP64 (numpy)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _resolve(film, fmt, param=0.0):
+    import torch
+    from spica_gb300 import gpu
+    dev = torch.from_numpy(np.ascontiguousarray(film, np.float32)).cuda()
+    return gpu.film_resolve(gpu.Context(0), dev, fmt, param).cpu().numpy()
+
+
+def _near(values, weight, ulps=(-3, -1, 0, 1, 3)):
+    """Film sums whose quotient by the weight lies on or a few float32 ulps beside the values."""
+    c = (np.asarray(values, np.float64) * weight).astype(np.float32)
+    return np.concatenate([c + np.float32(k) * np.spacing(c) for k in ulps])
+
+
+def _rows(sums, weight, rng):
+    """A film of one row: each sum as red, green and blue of some pixel."""
+    rgb = np.stack([sums, rng.permutation(sums), rng.permutation(sums)], 1).astype(np.float32)
+    return np.concatenate([rgb, np.full((rgb.shape[0], 1), weight, np.float32)], 1)[None]
+
+
+ODD_PIXELS = np.array([[0, 0, 0, 0], [0, 0, 0, 4], [1, 2, 3, 0], [1e-30, 0, 0, 1], [1e30, 1e20, 1, 1], [5, 5, 5, 1e-6],
+                       [17 * 16, 12 * 16, 4 * 16, 16], [1, 1, 1, 1], [3e38, 1, 0, 2], [0.5, 0.25, 0.125, 1],
+                       [-1, 2, 3, 1], [np.inf, 1, 2, 1], [1, np.nan, 2, 1], [1, 2, 3, 3e9]], np.float32)
+
+
+@pytest.mark.parametrize("gamma", [2.2, 1.0, 0.5, 0.02, 7.0])
+@pytest.mark.parametrize("weight", [1.0, 3.0, 16.0, 1000.5])
+def test_gamma_bytes_at_their_steps(gpulib, gamma, weight):
+    """Bytes of values on and beside every step (k / 255)^gamma, at random, and of pixels with
+    unusual weights and values: equal to the FP64 evaluation, save that a value within an ulp or
+    two of FP64 of a step may take either byte, as the two pow functions differ by that."""
+    from spica_gb300 import gpu
+    rng = np.random.default_rng(3)
+    steps = (np.arange(256) / 255.0) ** gamma
+    sums = np.concatenate([_near(steps, weight), (rng.random(5000) ** 3 * 1.5 * weight).astype(np.float32)])
+    film = np.concatenate([_rows(sums, weight, rng), ODD_PIXELS[None]], 1)
+    got = _resolve(film, gpu.FILM_GAMMA_BYTES, gamma).astype(int)
+    f = film.astype(np.float64)
+    with np.errstate(all="ignore"):
+        v = 255.0 * np.fmax(0.0, np.fmin(np.fmin(np.fmax((f[..., :3] / (f[..., 3:] + 1e-12)) ** (1.0 / gamma), 0.0),
+                                                 1.0), 1.0))
+    want = v.astype(int)
+    tie = np.abs(v - np.round(v)) < 255 * 2e-15
+    assert np.all((got == want) | (tie & (np.abs(got - want) <= 1))), np.argwhere(got != want)[:5]
+
+
+@pytest.mark.parametrize("weight", [1.0, 3.0, 16.0, 1000.5])
+def test_rgbe_at_its_steps(gpulib, weight):
+    """RGBE of values on and beside the mantissa steps and the exponents' limits, and of unusual
+    pixels, against HDRPixel in FP64 (core/image.cc:72-88)."""
+    from spica_gb300 import gpu
+    rng = np.random.default_rng(4)
+    values = np.concatenate([np.arange(1, 257) / 256.0, np.arange(1, 257) / 16.0, 2.0 ** np.arange(-30.0, 30.0)])
+    sums = np.concatenate([_near(values, weight), rng.lognormal(0, 3, 5000).astype(np.float32) * np.float32(weight)])
+    odd = ODD_PIXELS[np.isfinite(ODD_PIXELS).all(1) & (ODD_PIXELS >= 0).all(1)]
+    film = np.concatenate([_rows(sums, weight, rng), odd[None]], 1)
+    got = _resolve(film, gpu.FILM_RGBE)
+    c = film[..., :3].astype(np.float64) / (film[..., 3:].astype(np.float64) + 1e-12)
+    d = c.max(-1)
+    m, e = np.frexp(d)
+    with np.errstate(all="ignore"):
+        scale = np.where(d <= 1e-32, 0.0, m * 256.0 / d)
+    want = np.concatenate([(c * scale[..., None]).astype(np.uint8),
+                           np.where(d <= 1e-32, 0, e + 128).astype(np.uint8)[..., None]], -1)
+    np.testing.assert_array_equal(got, want)
