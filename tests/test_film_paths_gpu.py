@@ -69,3 +69,34 @@ def test_rgbe_at_its_steps(gpulib, weight):
     want = np.concatenate([(c * scale[..., None]).astype(np.uint8),
                            np.where(d <= 1e-32, 0, e + 128).astype(np.uint8)[..., None]], -1)
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("width, height", [(1, 1), (1, 9), (9, 1), (2, 2), (63, 65), (64, 64), (129, 5), (1920, 3),
+                                           (1921, 3), (3, 1921), (2100, 7), (5, 4000)])
+def test_durand_chunked_filter(gpulib, width, height):
+    """The line filter in chunks, and in tiles for lines longer than a block holds, against the
+    restatement's serial recursion (2e-6 relative, the float32 output's tolerance in
+    test_film_gpu.py)."""
+    from oracle import tmo_oracle
+    from spica_gb300 import gpu
+    rng = np.random.default_rng(width * 7 + height)
+    film = np.concatenate([rng.lognormal(0, 1.5, (height, width, 3)), np.full((height, width, 1), 4.0)], -1)
+    film = film.astype(np.float32)
+    film[rng.random((height, width)) < 0.05, :3] = 0.0
+    if width * height == 1:
+        film[...] = (1.0, 2.0, 3.0, 4.0)
+    got = _resolve(film, gpu.FILM_DURAND, 5.0)
+    with np.errstate(all="ignore"):
+        want = tmo_oracle.durand(film, 5.0)
+    np.testing.assert_allclose(got, want, rtol=2e-6, atol=1e-12)
+
+
+def test_durand_non_finite_pixel(gpulib):
+    """One infinite pixel: the recursion carries it to every pixel, and a NaN channel clamps to 0."""
+    from oracle import tmo_oracle
+    from spica_gb300 import gpu
+    film = np.ones((40, 50, 4), np.float32)
+    film[17, 49, 1] = np.inf
+    with np.errstate(all="ignore"):
+        want = tmo_oracle.durand(film, 5.0)
+    np.testing.assert_array_equal(_resolve(film, gpu.FILM_DURAND, 5.0), want)
