@@ -13,7 +13,7 @@
 //         mutual nearest neighbours merge into a new node, and the clusters are
 //         compacted in order, until one is left
 //   4. SAH-optimal choice of the wide tree, bottom-up over the clustering rounds
-//      (k_dp_round) -- the dynamic programme of Ylitie, Karras and Laine,
+//      (dpNode, with each round's new nodes) -- the dynamic programme of Ylitie, Karras and Laine,
 //      "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs"
 //      (HPG 2017): for every binary node, the least SAH cost of spreading 1..8
 //      child slots over its subtree, where a node is a leaf (at most 3 triangles),
@@ -26,12 +26,15 @@
 //      triangles are copied into leaf order as (v0, v1, v2) records.
 // The triangle set, and so the closest hit of every ray, is the reference's; only
 // the tree differs.  Its build is deterministic (no atomics decide structure).
+//
+// A build was bound by what surrounds its kernels: some 75 clustering rounds of eight launches
+// and a host round trip each, 30 allocations, and one thread per wide node in the collapse.  With
+// rounds that run ahead of the host, the last rounds in one block, one scratch allocation and
+// eight threads per wide node, 2.03M triangles take 11.4 -> 3.5 ms, 256 triangles 1.96 -> 0.28.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 #include <algorithm>
 #include <cstdio>
-#include <vector>
 
 #include "bvh.cuh"
 
@@ -51,7 +54,8 @@ __device__ __forceinline__ void atomicMaxFloat(float *a, float v) {
 }
 
 // scene bounds [0..5] and centroid bounds [6..11]
-__global__ void k_prim_bounds(const float *__restrict__ verts, int n, float *__restrict__ bounds) {
+constexpr int kBoundsBlock = 256;
+__global__ void __launch_bounds__(kBoundsBlock) k_prim_bounds(const float *__restrict__ verts, int n, float *__restrict__ bounds) {
     float lo[6], hi[6];
     for (int k = 0; k < 6; k++) {
         lo[k] = 3.0e38f;
@@ -75,13 +79,23 @@ __global__ void k_prim_bounds(const float *__restrict__ verts, int n, float *__r
             hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], off));
         }
     }
-    if ((threadIdx.x & 31) == 0) {
-        for (int a = 0; a < 3; a++) {
-            atomicMinFloat(&bounds[a], lo[a]);
-            atomicMaxFloat(&bounds[3 + a], hi[a]);
-            atomicMinFloat(&bounds[6 + a], lo[3 + a]);
-            atomicMaxFloat(&bounds[9 + a], hi[3 + a]);
+    // one update of the twelve bounds per block: all warps' updates of the same words would queue
+    __shared__ float part[kBoundsBlock / 32][12];
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0)
+        for (int k = 0; k < 6; k++) {
+            part[warp][k] = lo[k];
+            part[warp][6 + k] = hi[k];
         }
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        const int k = threadIdx.x;
+        float v = part[0][k];
+        for (int w = 1; w < kBoundsBlock / 32; w++) v = k < 6 ? fminf(v, part[w][k]) : fmaxf(v, part[w][k]);
+        // lo[0..2], lo[3..5] (centroids), hi[0..2], hi[3..5] go to 0..2, 6..8, 3..5, 9..11
+        const int at = (k % 6) % 3 + 3 * (k / 6) + 6 * ((k % 6) / 3);
+        if (k < 6) atomicMinFloat(&bounds[at], v);
+        else atomicMaxFloat(&bounds[at], v);
     }
 }
 
@@ -142,10 +156,11 @@ constexpr int kPlocBlock = 256;
 // at 1.0)
 constexpr float kCostNode = 1.0f, kCostTri = 1.0f;
 
-// per binary node: cost[8 * node + j - 1] = least SAH cost of its subtree over j child
-// slots; split[8 * node + j - 1] = slots given to the left child (0: the node itself
-// takes one slot); split of j = 8 before that choice is the node's own split as a wide
-// node (wideSplit); leaf[node]: the node itself is cheaper as a leaf than as a wide node
+// per inner binary node (ids 0..n-2): cost[8 * node + j - 1] = least SAH cost of its subtree
+// over j child slots; split[8 * node + j - 1] = slots given to the left child (0: the node
+// itself takes one slot); split of j = 8 before that choice is the node's own split as a wide
+// node (wideSplit); leaf[node]: the node itself is cheaper as a leaf than as a wide node.  A
+// triangle (ids n-1..) costs the same over any number of slots, which its box gives.
 struct DpArgs {
     float *cost;
     uint8_t *split;
@@ -154,35 +169,42 @@ struct DpArgs {
 };
 
 __global__ void k_leaf_bounds(const float *__restrict__ verts, const uint32_t *__restrict__ order, int n,
-                              float4 *bmin, float4 *bmax, int *count, int *clusters, DpArgs D) {
+                              float4 *bmin, float4 *bmax, int *count, int *clusters) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const float *v = verts + 9 * static_cast<int64_t>(order[j]);
     const int node = n - 1 + j;
-    const float4 lo = make_float4(fminf(v[0], fminf(v[3], v[6])), fminf(v[1], fminf(v[4], v[7])),
-                                  fminf(v[2], fminf(v[5], v[8])), 0.0f);
-    const float4 hi = make_float4(fmaxf(v[0], fmaxf(v[3], v[6])), fmaxf(v[1], fmaxf(v[4], v[7])),
-                                  fmaxf(v[2], fmaxf(v[5], v[8])), 0.0f);
-    bmin[node] = lo;
-    bmax[node] = hi;
+    bmin[node] = make_float4(fminf(v[0], fminf(v[3], v[6])), fminf(v[1], fminf(v[4], v[7])),
+                             fminf(v[2], fminf(v[5], v[8])), 0.0f);
+    bmax[node] = make_float4(fmaxf(v[0], fmaxf(v[3], v[6])), fmaxf(v[1], fmaxf(v[4], v[7])),
+                             fmaxf(v[2], fmaxf(v[5], v[8])), 0.0f);
     count[node] = 1;
     clusters[j] = node;
-    const float2 dx = make_float2(hi.x - lo.x, hi.y - lo.y);
-    const float c = kCostTri * 2.0f * (dx.x * dx.y + dx.y * (hi.z - lo.z) + (hi.z - lo.z) * dx.x);
-    for (int k = 0; k < 8; k++) {
-        D.cost[8 * static_cast<int64_t>(node) + k] = c;
-        D.split[8 * static_cast<int64_t>(node) + k] = 0;
-    }
-    D.leaf[node] = 1;
 }
+
+// The clustering runs ahead of the host: round r reads its cluster count m and the next free
+// node id top from rounds[r] and leaves the next round's in rounds[r + 1], so the host launches
+// kRoundsAhead rounds, sized by the last count it knows, between two looks.  From kTailClusters
+// clusters on, one block does the rest (k_ploc_tail): with 4096 / 2048 / 1024 / 512 of them the
+// 2M-triangle build takes 3.50 / 3.48 / 3.47 / 3.60 ms, 16k triangles 1.12 / 1.08 / 1.10 / 1.16.
+struct RoundState {
+    int m, top;
+};
+constexpr int kRoundsAhead = 4;
+constexpr int kMaxRounds = 1024;
+constexpr int kTailClusters = 2048;
+constexpr int kMergeBlock = 1024;
 
 // nearest neighbour of each cluster: least surface area of the merged box among the
 // clusters within kPlocRadius positions (ties: the lower position); the window's boxes
 // are staged in shared memory
-__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const int *__restrict__ clusters, int m,
+__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const int *__restrict__ clusters,
+                                                        const RoundState *__restrict__ round,
                                                         const float4 *__restrict__ bmin,
                                                         const float4 *__restrict__ bmax, int *nn) {
     __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius], shi[kPlocBlock + 2 * kPlocRadius];
+    const int m = round->m;
+    if (m <= kTailClusters || static_cast<int>(blockIdx.x) * kPlocBlock >= m) return;
     const int base = blockIdx.x * kPlocBlock - kPlocRadius;
     for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock) {
         const int p = base + k;
@@ -213,29 +235,93 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const int *__restrict__ 
     nn[i] = bestJ;
 }
 
-// a cluster leads a merge when it and its neighbour chose each other and it comes
-// first; it survives the round unless it is the second of such a pair
-__global__ void k_ploc_flags(const int *__restrict__ nn, int m, int *lead, int *keep) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int j = nn[i];
+// A cluster leads a merge when it and its neighbour chose each other and it comes first; it
+// survives the round unless it is the second of such a pair.
+__device__ __forceinline__ void mergeFlags(const int *nn, int i, int m, bool *lead, bool *keep) {
+    const int j = i < m ? nn[i] : -1;
     const bool mutual = j >= 0 && nn[j] == i;
-    lead[i] = mutual && i < j ? 1 : 0;
-    keep[i] = mutual && i > j ? 0 : 1;
+    *lead = mutual && i < j;
+    *keep = i < m && !(mutual && i > j);
+}
+// exclusive counts of the block's flags before this thread (lead | keep << 16), and the block's
+// totals; called by all threads of a block of kMergeBlock
+__device__ __forceinline__ uint32_t countBefore(bool lead, bool keep, uint32_t *warpSum, uint32_t *total) {
+    const unsigned lb = __ballot_sync(0xffffffffu, lead), kb = __ballot_sync(0xffffffffu, keep);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    if (lane == 0) warpSum[warp] = static_cast<uint32_t>(__popc(lb)) | static_cast<uint32_t>(__popc(kb)) << 16;
+    __syncthreads();
+    // every warp scans the warps' sums for itself
+    const uint32_t mine = warpSum[lane];
+    uint32_t sum = mine;
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, sum, off);
+        if (lane >= off) sum += v;
+    }
+    *total = __shfl_sync(0xffffffffu, sum, 31);
+    const uint32_t before = __shfl_sync(0xffffffffu, sum - mine, warp);
+    return before + (static_cast<uint32_t>(__popc(lb & below)) | static_cast<uint32_t>(__popc(kb & below)) << 16);
+}
+static_assert(kMergeBlock == 1024, "32 warps, a lane for each in countBefore; counts of 16 bits");
+
+// leads and survivors of each block of kMergeBlock clusters
+__global__ void __launch_bounds__(kMergeBlock) k_ploc_count(const int *__restrict__ nn,
+                                                            const RoundState *__restrict__ round, uint32_t *sums) {
+    __shared__ uint32_t warpSum[32];
+    const int m = round->m;
+    if (m <= kTailClusters || static_cast<int>(blockIdx.x) * kMergeBlock >= m) return;
+    bool lead, keep;
+    mergeFlags(nn, blockIdx.x * kMergeBlock + threadIdx.x, m, &lead, &keep);
+    uint32_t total;
+    countBefore(lead, keep, warpSum, &total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// merged nodes take ids top - leadOffset (descending, so the last merge, the root, is
-// node 0); survivors are compacted in order
-__global__ void k_ploc_merge(const int *__restrict__ clusters, int m, const int *__restrict__ nn,
-                             const int *__restrict__ lead, const int *__restrict__ leadOff,
-                             const int *__restrict__ keep, const int *__restrict__ keepOff, int top, int2 *child,
-                             float4 *bmin, float4 *bmax, int *count, int *next) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m || !keep[i]) return;
+// merged nodes take ids top - (leads before) (descending, so the last merge, the root, is node
+// 0); survivors are compacted in order.  Each block adds up the counts of the blocks before it.
+__global__ void __launch_bounds__(kMergeBlock) k_ploc_merge(const int *__restrict__ clusters, RoundState *round,
+                                                            const int *__restrict__ nn,
+                                                            const uint32_t *__restrict__ sums, int2 *child,
+                                                            float4 *bmin, float4 *bmax, int *count, int *next) {
+    __shared__ uint32_t warpSum[32];
+    __shared__ int base[2];
+    const int m = round->m, top = round->top;
+    if (static_cast<int>(blockIdx.x) * kMergeBlock >= m) return;
+    if (m <= kTailClusters) {   // nothing left for the rounds: clusters and state go on to the tail
+        const int i = blockIdx.x * kMergeBlock + threadIdx.x;
+        if (i < m) next[i] = clusters[i];
+        if (i == 0) round[1] = round[0];
+        return;
+    }
+    if (threadIdx.x < 2) base[threadIdx.x] = 0;
+    __syncthreads();
+    int lsum = 0, ksum = 0;
+    for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += kMergeBlock) {
+        lsum += sums[b] & 0xFFFFu;
+        ksum += sums[b] >> 16;
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        lsum += __shfl_xor_sync(0xffffffffu, lsum, off);
+        ksum += __shfl_xor_sync(0xffffffffu, ksum, off);
+    }
+    if ((threadIdx.x & 31) == 0 && (lsum | ksum)) {
+        atomicAdd(&base[0], lsum);
+        atomicAdd(&base[1], ksum);
+    }
+    const int i = blockIdx.x * kMergeBlock + threadIdx.x;
+    bool lead, keep;
+    mergeFlags(nn, i, m, &lead, &keep);
+    uint32_t total;
+    const uint32_t before = countBefore(lead, keep, warpSum, &total);   // synchronises: base is complete
+    if (threadIdx.x == 0 && (blockIdx.x + 1) * kMergeBlock >= static_cast<unsigned>(m)) {
+        round[1].m = base[1] + static_cast<int>(total >> 16);
+        round[1].top = top - base[0] - static_cast<int>(total & 0xFFFFu);
+    }
+    if (!keep) return;
     int node = clusters[i];
-    if (lead[i]) {
+    if (lead) {
         const int a = node, b = clusters[nn[i]];
-        const int id = top - leadOff[i];
+        const int id = top - base[0] - static_cast<int>(before & 0xFFFFu);
         child[id] = make_int2(a, b);
         const float4 a0 = bmin[a], a1 = bmax[a], b0 = bmin[b], b1 = bmax[b];
         bmin[id] = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.0f);
@@ -243,25 +329,43 @@ __global__ void k_ploc_merge(const int *__restrict__ clusters, int m, const int 
         count[id] = count[a] + count[b];
         node = id;
     }
-    next[keepOff[i]] = node;
+    next[base[1] + static_cast<int>(before >> 16)] = node;
 }
 
-
-// one clustering round's nodes (ids lo..hi; their children are from earlier rounds)
-__global__ void k_dp_round(const int2 *__restrict__ child, const int *__restrict__ count,
-                           const float4 *__restrict__ bmin, const float4 *__restrict__ bmax, int lo, int hi,
-                           DpArgs D, int kLeafLimit) {
-    const int id = lo + blockIdx.x * blockDim.x + threadIdx.x;
-    if (id > hi) return;
-    const int2 c = child[id];
-    const float *CL = D.cost + 8 * static_cast<int64_t>(c.x), *CR = D.cost + 8 * static_cast<int64_t>(c.y);
+// the SAH programme of one node, from its children's (n: triangles of the scene)
+__device__ __forceinline__ void dpNode(const DpArgs &D, int n, int id, int2 c, int triangles, float4 lo, float4 hi,
+                                       const float4 *bmin, const float4 *bmax) {
+    float CL[7], CR[7];
+    auto load = [&](int x, float *C) {
+        if (x >= n - 1) {
+            const float4 l = bmin[x], h = bmax[x];
+            const float2 dx = make_float2(h.x - l.x, h.y - l.y);
+            const float v = kCostTri * 2.0f * (dx.x * dx.y + dx.y * (h.z - l.z) + (h.z - l.z) * dx.x);
+#pragma unroll
+            for (int k = 0; k < 7; k++) C[k] = v;
+        } else {
+            const float4 *p = reinterpret_cast<const float4 *>(D.cost + 8 * static_cast<int64_t>(x));
+            const float4 a = p[0], b = p[1];
+            C[0] = a.x;
+            C[1] = a.y;
+            C[2] = a.z;
+            C[3] = a.w;
+            C[4] = b.x;
+            C[5] = b.y;
+            C[6] = b.z;
+        }
+    };
+    load(c.x, CL);
+    load(c.y, CR);
     float S[9];
     uint8_t K[9];
     S[1] = 3.0e38f;
     K[1] = 0;
+#pragma unroll
     for (int j = 2; j <= 8; j++) {
         float best = 3.0e38f;
         uint8_t bk = 1;
+#pragma unroll
         for (int k = 1; k < j; k++) {
             const float v = CL[k - 1] + CR[j - k - 1];
             if (v < best) {
@@ -276,22 +380,141 @@ __global__ void k_dp_round(const int2 *__restrict__ child, const int *__restrict
             K[j] = K[j - 1];
         }
     }
-    const float A = areaOf(bmin[id], bmax[id]);
+    const float A = areaOf(lo, hi);
     const float cInternal = kCostNode * A + S[8];
-    const float cLeaf = count[id] <= kLeafLimit ? kCostTri * A * static_cast<float>(count[id]) : 3.0e38f;
+    const float cLeaf = triangles <= kLeafMax ? kCostTri * A * static_cast<float>(triangles) : 3.0e38f;
     const bool asLeaf = cLeaf <= cInternal;
     const float C = asLeaf ? cLeaf : cInternal;
-    float *out = D.cost + 8 * static_cast<int64_t>(id);
-    uint8_t *sp = D.split + 8 * static_cast<int64_t>(id);
+    float out[8];
+    uint32_t sp[2] = {0u, 0u};
     out[0] = C;
-    sp[0] = 0;
+#pragma unroll
     for (int j = 2; j <= 8; j++) {
         const bool self = C <= S[j];
         out[j - 1] = self ? C : S[j];
-        sp[j - 1] = self ? 0 : K[j];
+        if (!self) sp[(j - 1) >> 2] |= static_cast<uint32_t>(K[j]) << (8 * ((j - 1) & 3));
     }
+    float4 *o = reinterpret_cast<float4 *>(D.cost + 8 * static_cast<int64_t>(id));
+    o[0] = make_float4(out[0], out[1], out[2], out[3]);
+    o[1] = make_float4(out[4], out[5], out[6], out[7]);
+    reinterpret_cast<uint2 *>(D.split)[id] = make_uint2(sp[0], sp[1]);
     D.wideSplit[id] = K[8];
     D.leaf[id] = asLeaf ? 1 : 0;
+}
+
+// one clustering round's nodes (round[1].top < id <= round[0].top; their children are from
+// earlier rounds)
+__global__ void k_dp_round(const int2 *__restrict__ child, const int *__restrict__ count,
+                           const float4 *__restrict__ bmin, const float4 *__restrict__ bmax,
+                           const RoundState *__restrict__ round, int n, DpArgs D) {
+    const int id = round[1].top + 1 + static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    if (id > round[0].top) return;
+    dpNode(D, n, id, child[id], count[id], bmin[id], bmax[id], bmin, bmax);
+}
+
+// The clustering's last rounds, with their SAH programme, in one block: at most kTailClusters
+// clusters, whose boxes stay in shared memory.  A round of a few thousand clusters is too little
+// for the chip and its launches cost more than its work; there are some forty of them.
+// state: in, the clusters and next free id; out, what is left (one cluster, top -1).
+constexpr int kTailSmem = kTailClusters * (2 * static_cast<int>(sizeof(float4)) + static_cast<int>(sizeof(int)));
+__global__ void __launch_bounds__(kMergeBlock) k_ploc_tail(const int *__restrict__ clusters, RoundState *state,
+                                                           int2 *child, float4 *bmin, float4 *bmax, int *count, int n,
+                                                           DpArgs D) {
+    extern __shared__ float4 box[];   // per cluster: lo (w: node id), hi (w: triangles)
+    __shared__ uint32_t warpSum[32];
+    float4 *slo = box, *shi = box + kTailClusters;
+    int *nn = reinterpret_cast<int *>(shi + kTailClusters);
+    int m = state->m, top = state->top;
+    if (m > kTailClusters) return;
+    const int t = threadIdx.x;
+    for (int i = t; i < m; i += kMergeBlock) {
+        const int c = clusters[i];
+        float4 lo = bmin[c], hi = bmax[c];
+        lo.w = __int_as_float(c);
+        hi.w = __int_as_float(count[c]);
+        slo[i] = lo;
+        shi[i] = hi;
+    }
+    __syncthreads();
+    while (m > 1) {
+        // nearest neighbours as in k_ploc_nn; few clusters share the block's threads, P to a
+        // cluster, each over every P-th position of the window
+        int P = 1;
+        while (P < 32 && 2 * P * m <= kMergeBlock) P *= 2;
+        for (int w = t; w < (m * P + 31) / 32 * 32; w += kMergeBlock) {   // whole warps
+            const int i = min(w / P, m - 1);
+            const float4 lo = slo[i], hi = shi[i];
+            float best = 3.0e38f;
+            int bestJ = -1;
+            const int j1 = min(i + kPlocRadius, m - 1);
+            for (int j = max(i - kPlocRadius, 0) + w % P; j <= j1; j += P) {
+                if (j == i) continue;
+                const float4 a = slo[j], b = shi[j];
+                const float area = areaOf(make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), 0.0f),
+                                          make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), 0.0f));
+                if (area < best) {
+                    best = area;
+                    bestJ = j;
+                }
+            }
+            for (int off = 1; off < P; off <<= 1) {   // the least area, the lowest position of equals
+                const float a2 = __shfl_xor_sync(0xffffffffu, best, off);
+                const int j2 = __shfl_xor_sync(0xffffffffu, bestJ, off);
+                if (j2 >= 0 && (bestJ < 0 || a2 < best || (a2 == best && j2 < bestJ))) {
+                    best = a2;
+                    bestJ = j2;
+                }
+            }
+            if (w < m * P && w % P == 0) nn[i] = bestJ;
+        }
+        __syncthreads();
+        // merge and compact, a block's width of clusters at a time; a tile writes only positions
+        // at or before its own clusters, once all of them are read
+        int merges = 0, kept = 0;
+        for (int base = 0; base < m; base += kMergeBlock) {
+            const int i = base + t;
+            bool lead, keep;
+            mergeFlags(nn, i, m, &lead, &keep);
+            uint32_t total;
+            const uint32_t before = countBefore(lead, keep, warpSum, &total);
+            float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+            if (keep) {
+                lo = slo[i];
+                hi = shi[i];
+                if (lead) {
+                    const float4 l2 = slo[nn[i]], h2 = shi[nn[i]];
+                    const int a = __float_as_int(lo.w), b = __float_as_int(l2.w);
+                    const int triangles = __float_as_int(hi.w) + __float_as_int(h2.w);
+                    const int id = top - merges - static_cast<int>(before & 0xFFFFu);
+                    lo = make_float4(fminf(lo.x, l2.x), fminf(lo.y, l2.y), fminf(lo.z, l2.z), 0.0f);
+                    hi = make_float4(fmaxf(hi.x, h2.x), fmaxf(hi.y, h2.y), fmaxf(hi.z, h2.z), 0.0f);
+                    child[id] = make_int2(a, b);
+                    bmin[id] = lo;
+                    bmax[id] = hi;
+                    count[id] = triangles;
+                    dpNode(D, n, id, make_int2(a, b), triangles, lo, hi, bmin, bmax);
+                    lo.w = __int_as_float(id);
+                    hi.w = __int_as_float(triangles);
+                }
+            }
+            __syncthreads();
+            if (keep) {
+                const int at = kept + static_cast<int>(before >> 16);
+                slo[at] = lo;
+                shi[at] = hi;
+            }
+            merges += static_cast<int>(total & 0xFFFFu);
+            kept += static_cast<int>(total >> 16);
+            __syncthreads();
+        }
+        if (merges == 0) break;   // reported by the host: clusters are left
+        top -= merges;
+        m = kept;
+    }
+    if (t == 0) {
+        state[1].m = m;
+        state[1].top = top;
+    }
 }
 
 struct CollapseArgs {
@@ -308,188 +531,228 @@ struct CollapseArgs {
     WideNode *nodes;
     TriRecord *tris;
     int2 *slot_shade;
-    int *counters;   // [0] wide nodes allocated, [1] triangles placed, [2] next-level items
+    unsigned long long *level;   // per level: wide nodes (low half) and triangles (high half) it allocated
 };
 
-// the triangles (code-order positions) under binary node b, at most kLeafMax of them,
-// left subtree first
-__device__ __forceinline__ int leafPrims(const CollapseArgs &A, int b, int *pos) {
-    int stack[2 * kLeafMax], sp = 0, k = 0;
-    stack[sp++] = b;
-    while (sp > 0 && k < kLeafMax) {
-        const int x = stack[--sp];
-        if (x >= A.n - 1) {
-            pos[k++] = x - (A.n - 1);
-        } else if (sp + 2 <= 2 * kLeafMax) {
-            const int2 c = A.child[x];
-            stack[sp++] = c.y;
-            stack[sp++] = c.x;
-        }
-    }
-    return k;
+__device__ __forceinline__ float groupMin(float v) {
+    for (int off = 1; off < 8; off <<= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
+__device__ __forceinline__ float groupMax(float v) {
+    for (int off = 1; off < 8; off <<= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
+    return v;
+}
+__device__ __forceinline__ uint32_t groupOr(uint32_t v) {
+    for (int off = 1; off < 8; off <<= 1) v |= __shfl_xor_sync(0xffffffffu, v, off);
+    return v;
 }
 
-// one thread per wide node of the current level; items are (binary node, wide node)
-__global__ void k_collapse(CollapseArgs A, const int2 *__restrict__ items, int nitems, int2 *__restrict__ next) {
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= nitems) return;
-    const int b = items[it].x, w = items[it].y;
-    const bool rootLeaf = b >= A.n - 1;   // single-triangle scene
-    int C[8];
-    int nc = 0;
-    if (rootLeaf) {
-        C[nc++] = b;
-    } else {
-        // the 8 slots of wide node b, spread as the SAH programme decided: (node, slots)
-        int stN[8], stJ[8], sp = 0;
-        const int k0 = A.dp.wideSplit[b];
-        stN[sp] = A.child[b].y;
-        stJ[sp++] = 8 - k0;
-        stN[sp] = A.child[b].x;
-        stJ[sp++] = k0;
-        while (sp > 0 && nc < 8) {
-            const int x = stN[--sp], j = stJ[sp];
-            const int k = (x < A.n - 1 && j > 1) ? A.dp.split[8 * static_cast<int64_t>(x) + j - 1] : 0;
-            if (k == 0 || sp + 2 > 8) {
-                C[nc++] = x;
-            } else {
-                const int2 cc = A.child[x];
-                stN[sp] = cc.y;
-                stJ[sp++] = j - k;
-                stN[sp] = cc.x;
-                stJ[sp++] = k;
-            }
-        }
+// One level of the wide tree, eight threads per wide node (a thread per child, then per slot);
+// items are (binary node, wide node), a level's items in the order its parents allocated them.
+// Its levels are few and the upper ones small, so a level costs the latency of one node: with
+// a thread per node that was the greedy assignment over a local 8 x 8 table and 48 FP64
+// divisions (73 us for the 5 nodes of the box room); here each thread keeps its child's eight
+// costs in registers, planes are quantised exactly in float32 with directed rounding, and the
+// allocations of a block's 16 nodes take one atomic instead of 48.
+constexpr int kCollapseBlock = 128, kCollapseNodes = kCollapseBlock / 8;
+__global__ void __launch_bounds__(kCollapseBlock) k_collapse(CollapseArgs A, int levelIdx,
+                                                             const int2 *__restrict__ items, int2 *__restrict__ next) {
+    __shared__ unsigned long long alloc[kCollapseNodes];
+    // nodes and triangles placed by the levels before this one; this level's items
+    int nodeBase = 1, triBase0 = 0;
+    for (int l = 0; l < levelIdx; l++) {
+        nodeBase += static_cast<int>(A.level[l] & 0xFFFFFFFFull);
+        triBase0 += static_cast<int>(A.level[l] >> 32);
     }
-    // node box
-    float3 lo = mk(3.0e38f, 3.0e38f, 3.0e38f), hi = mk(-3.0e38f, -3.0e38f, -3.0e38f);
-    for (int k = 0; k < nc; k++) {
-        lo = fminf3(lo, xyz(A.bmin[C[k]]));
-        hi = fmaxf3(hi, xyz(A.bmax[C[k]]));
-    }
-    const float3 ctr = (lo + hi) * 0.5f;
-    // greedy slot assignment: child whose centroid offset lies in octant o prefers slot o
-    int slotOf[8];
-    bool usedSlot[8] = {false, false, false, false, false, false, false, false};
-    bool done[8] = {false, false, false, false, false, false, false, false};
-    float cost[8][8];
-    for (int k = 0; k < nc; k++) {
-        const float3 c = (xyz(A.bmin[C[k]]) + xyz(A.bmax[C[k]])) * 0.5f - ctr;
-        for (int s = 0; s < 8; s++) {
-            const float3 sg = mk((s & 1) ? -1.0f : 1.0f, (s & 2) ? -1.0f : 1.0f, (s & 4) ? -1.0f : 1.0f);
-            cost[k][s] = -dot(c, sg);
-        }
-    }
-    for (int r = 0; r < nc; r++) {
-        float bc = 3.0e38f;
-        int bk = -1, bs = -1;
-        for (int k = 0; k < nc; k++) {
-            if (done[k]) continue;
-            for (int s = 0; s < 8; s++) {
-                if (usedSlot[s]) continue;
-                if (cost[k][s] < bc) {
-                    bc = cost[k][s];
-                    bk = k;
-                    bs = s;
+    const int nitems = levelIdx == 0 ? 1 : static_cast<int>(A.level[levelIdx - 1] & 0xFFFFFFFFull);
+    const int lane = threadIdx.x & 31, sub = lane & 7, group = threadIdx.x >> 3;
+    const unsigned groupShift = static_cast<unsigned>(lane & 24);
+    for (int tile = blockIdx.x * kCollapseNodes; tile < nitems; tile += gridDim.x * kCollapseNodes) {
+        const bool live = tile + group < nitems;
+        const int2 item = live ? items[tile + group] : make_int2(A.n - 1, 0);
+        // the eight slots of the wide node spread over its subtree as the SAH programme decided:
+        // thread s follows the part that slot s belongs to, [start, start + slots)
+        int x = item.x, start = 0, slots = 8;
+        {
+            int k = x < A.n - 1 ? A.dp.wideSplit[x] : 0;   // 0: a single-triangle scene's root
+            while (__any_sync(0xffffffffu, k != 0)) {
+                if (k != 0) {
+                    const int2 c = A.child[x];
+                    if (sub - start < k) {
+                        x = c.x;
+                        slots = k;
+                    } else {
+                        x = c.y;
+                        start += k;
+                        slots -= k;
+                    }
+                    k = x < A.n - 1 && slots > 1 ? A.dp.split[8 * static_cast<int64_t>(x) + slots - 1] : 0;
                 }
             }
         }
-        done[bk] = true;
-        usedSlot[bs] = true;
-        slotOf[bk] = bs;
-    }
-    // classify children: internal (wide node) or leaf (<= 3 triangles)
-    int slotChild[8];
-    for (int s = 0; s < 8; s++) slotChild[s] = -1;
-    for (int k = 0; k < nc; k++) slotChild[slotOf[k]] = C[k];
-    uint32_t imask = 0;
-    int nInt = 0, nTri = 0;
-    for (int s = 0; s < 8; s++) {
-        const int c = slotChild[s];
-        if (c < 0) continue;
-        const int count = A.count[c];
-        if (c < A.n - 1 && (count > kLeafMax || !A.dp.leaf[c])) {
-            imask |= 1u << s;
-            nInt++;
-        } else {
-            nTri += count;
+        const bool isChild = live && sub == start;   // children in the order of their slots, left first
+        const unsigned childMask = (__ballot_sync(0xffffffffu, isChild) >> groupShift) & 0xFFu;
+        const int nc = __popc(childMask);
+        const float4 cl = isChild ? A.bmin[x] : make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f);
+        const float4 ch = isChild ? A.bmax[x] : make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
+        const float3 lo = mk(groupMin(cl.x), groupMin(cl.y), groupMin(cl.z));
+        const float3 hi = mk(groupMax(ch.x), groupMax(ch.y), groupMax(ch.z));
+        const float3 ctr = (lo + hi) * 0.5f;
+        const float3 c = (xyz(cl) + xyz(ch)) * 0.5f - ctr;
+        // greedy slot assignment: child whose centroid offset lies in octant o prefers slot o;
+        // the cheapest pair of an unplaced child and a free slot first (ties: the first child,
+        // then the first slot)
+        float cost[8];
+#pragma unroll
+        for (int s = 0; s < 8; s++)
+            cost[s] = -(((s & 1) ? -c.x : c.x) + ((s & 2) ? -c.y : c.y) + ((s & 4) ? -c.z : c.z));
+        uint32_t used = 0u;
+        int slot = -1;
+        const int rounds = __reduce_max_sync(0xffffffffu, nc);
+        for (int r = 0; r < rounds; r++) {
+            float bc = 3.0e38f;
+            int bs = -1;
+#pragma unroll
+            for (int s = 0; s < 8; s++)
+                if (!((used >> s) & 1u) && (cost[s] < bc || bs < 0)) {
+                    bc = cost[s];
+                    bs = s;
+                }
+            const bool open = isChild && slot < 0 && r < nc;
+            float v = open ? bc : INFINITY;
+            int who = open ? sub : 8 + sub;
+            for (int off = 1; off < 8; off <<= 1) {
+                const float v2 = __shfl_xor_sync(0xffffffffu, v, off);
+                const int who2 = __shfl_xor_sync(0xffffffffu, who, off);
+                if ((who2 < 8 && who >= 8) || ((who2 < 8) == (who < 8) && (v2 < v || (!(v < v2) && who2 < who)))) {
+                    v = v2;
+                    who = who2;
+                }
+            }
+            const int taken = __shfl_sync(0xffffffffu, bs, static_cast<int>(groupShift) + (who & 7));
+            if (who < 8) {
+                used |= 1u << taken;
+                if (sub == who) slot = taken;
+            }
         }
-    }
-    const int childBase = nInt ? atomicAdd(&A.counters[0], nInt) : 0;
-    const int triBase = nTri ? atomicAdd(&A.counters[1], nTri) : 0;
-    const int itemBase = nInt ? atomicAdd(&A.counters[2], nInt) : 0;
+        // the threads without a child take the free slots, which stay empty
+        if (slot < 0) slot = static_cast<int>(__fns(~used & 0xFFu, 0, __popc(~childMask & ((1u << sub) - 1u) & 0xFFu) + 1)) & 7;
+        // children: internal (wide node) or leaf (<= 3 triangles)
+        const int triangles = isChild ? A.count[x] : 0;
+        const bool inner = isChild && x < A.n - 1 && (triangles > kLeafMax || !A.dp.leaf[x]);
+        const int leafTris = isChild && !inner ? triangles : 0;
+        const uint32_t imask = groupOr(inner ? 1u << slot : 0u);
+        const uint32_t tri2 = groupOr(static_cast<uint32_t>(leafTris) << (2 * slot));   // 2 bits per slot
+        const int nInt = __popc(imask), nTri = __popc(tri2 & 0x5555u) + 2 * __popc(tri2 & 0xAAAAu);
+        const uint32_t triBelow = tri2 & ((1u << (2 * slot)) - 1u);
+        const int triOff = __popc(triBelow & 0x5555u) + 2 * __popc(triBelow & 0xAAAAu);
+        const int rank = __popc(imask & ((1u << slot) - 1u));
+        if (sub == 0) alloc[group] = static_cast<unsigned long long>(nInt) | static_cast<unsigned long long>(nTri) << 32;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long sum = 0;
+            for (int g = 0; g < kCollapseNodes; g++) {
+                const unsigned long long v = alloc[g];
+                alloc[g] = sum;
+                sum += v;
+            }
+            const unsigned long long at = sum ? atomicAdd(&A.level[levelIdx], sum) : 0ull;
+            for (int g = 0; g < kCollapseNodes; g++) alloc[g] += at;
+        }
+        __syncthreads();
+        const int levelOff = static_cast<int>(alloc[group] & 0xFFFFFFFFull);   // among this level's new nodes
+        const int childBase = nInt ? nodeBase + levelOff : 0;
+        const int triBase = nTri ? triBase0 + static_cast<int>(alloc[group] >> 32) : 0;
+        __syncthreads();   // alloc is read: the next tile may overwrite it
 
-    WideNode node;
-    node.px = lo.x;
-    node.py = lo.y;
-    node.pz = lo.z;
-    int e[3];
-    const float ext[3] = {hi.x - lo.x, hi.y - lo.y, hi.z - lo.z};
-    for (int a = 0; a < 3; a++) {
-        int ex = -126;
-        if (ext[a] > 0.0f) {
-            frexpf(ext[a] / 255.0f, &ex);   // ext/255 = m 2^ex, m in [0.5, 1)
-            ex = max(ex, -126);
-            for (int g = 0; g < 4 && ldexpf(255.0f, ex) < ext[a]; g++) ex++;
-        }
-        e[a] = ex;
-    }
-    node.ex = static_cast<uint8_t>(e[0] + 127);
-    node.ey = static_cast<uint8_t>(e[1] + 127);
-    node.ez = static_cast<uint8_t>(e[2] + 127);
-    node.imask = static_cast<uint8_t>(imask);
-    node.child_base = static_cast<uint32_t>(childBase);
-    node.tri_base = static_cast<uint32_t>(triBase);
-    const double p[3] = {lo.x, lo.y, lo.z};
-    int rank = 0, triOff = 0;
-    for (int s = 0; s < 8; s++) {
-        const int c = slotChild[s];
-        if (c < 0) {
-            node.meta[s] = 0;
-            node.qlo_x[s] = node.qlo_y[s] = node.qlo_z[s] = 0;
-            node.qhi_x[s] = node.qhi_y[s] = node.qhi_z[s] = 0;
-            continue;
-        }
-        const float4 cl = A.bmin[c], ch = A.bmax[c];
-        const double clo[3] = {cl.x, cl.y, cl.z}, chi[3] = {ch.x, ch.y, ch.z};
-        uint8_t ql[3], qh[3];
+        int e[3];
+        const float ext[3] = {hi.x - lo.x, hi.y - lo.y, hi.z - lo.z};
+#pragma unroll
         for (int a = 0; a < 3; a++) {
-            const double sc = ldexp(1.0, e[a]);
-            double l = floor((clo[a] - p[a]) / sc), h = ceil((chi[a] - p[a]) / sc);
-            l = fmin(fmax(l, 0.0), 255.0);
-            h = fmin(fmax(h, 0.0), 255.0);
-            ql[a] = static_cast<uint8_t>(l);
-            qh[a] = static_cast<uint8_t>(h);
+            int ex = -126;
+            if (ext[a] > 0.0f) {
+                frexpf(ext[a] / 255.0f, &ex);   // ext/255 = m 2^ex, m in [0.5, 1)
+                ex = max(ex, -126);
+                for (int g = 0; g < 4 && ldexpf(255.0f, ex) < ext[a]; g++) ex++;
+            }
+            e[a] = ex;
         }
-        node.qlo_x[s] = ql[0];
-        node.qlo_y[s] = ql[1];
-        node.qlo_z[s] = ql[2];
-        node.qhi_x[s] = qh[0];
-        node.qhi_y[s] = qh[1];
-        node.qhi_z[s] = qh[2];
-        if (imask & (1u << s)) {
-            node.meta[s] = static_cast<uint8_t>(0x20 | (24 + s));
-            next[itemBase + rank] = make_int2(c, childBase + rank);
-            rank++;
-        } else {
-            int pos[kLeafMax];
-            const int count = leafPrims(A, c, pos);
-            node.meta[s] = static_cast<uint8_t>((((1u << count) - 1u) << 5) | static_cast<uint32_t>(triOff));
-            for (int q = 0; q < count; q++) {
-                const uint32_t prim = A.order[pos[q]];
-                const float *v = A.verts + 9 * static_cast<int64_t>(prim);
+        if (!live) continue;
+        WideNode &node = A.nodes[item.y];
+        if (sub == 0) {
+            node.px = lo.x;
+            node.py = lo.y;
+            node.pz = lo.z;
+            *reinterpret_cast<uint32_t *>(&node.ex) =
+                static_cast<uint32_t>(static_cast<uint8_t>(e[0] + 127)) |
+                static_cast<uint32_t>(static_cast<uint8_t>(e[1] + 127)) << 8 |
+                static_cast<uint32_t>(static_cast<uint8_t>(e[2] + 127)) << 16 | imask << 24;
+            node.child_base = static_cast<uint32_t>(childBase);
+            node.tri_base = static_cast<uint32_t>(triBase);
+        }
+        // floor and ceiling of (bound - origin) / 2^e in real arithmetic: every k 2^e with k <=
+        // 255 is a float, so rounding the difference towards it does not pass an integer, and
+        // the scaling is exact (an underflow to 0 keeps a ceiling of 1)
+        uint8_t ql[3] = {0, 0, 0}, qh[3] = {0, 0, 0};
+        uint8_t meta = 0;
+        if (isChild) {
+            const float p[3] = {lo.x, lo.y, lo.z}, b0[3] = {cl.x, cl.y, cl.z}, b1[3] = {ch.x, ch.y, ch.z};
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                const float down = __fsub_rd(b0[a], p[a]), up = __fsub_ru(b1[a], p[a]);
+                const float l = floorf(ldexpf(down, -e[a]));
+                float h = ceilf(ldexpf(up, -e[a]));
+                if (up > 0.0f && h < 1.0f) h = 1.0f;
+                ql[a] = static_cast<uint8_t>(fminf(fmaxf(l, 0.0f), 255.0f));
+                qh[a] = static_cast<uint8_t>(fminf(fmaxf(h, 0.0f), 255.0f));
+            }
+            meta = inner ? static_cast<uint8_t>(0x20 | (24 + slot))
+                         : static_cast<uint8_t>((((1u << leafTris) - 1u) << 5) | static_cast<uint32_t>(triOff));
+        }
+        node.meta[slot] = meta;
+        node.qlo_x[slot] = ql[0];
+        node.qlo_y[slot] = ql[1];
+        node.qlo_z[slot] = ql[2];
+        node.qhi_x[slot] = qh[0];
+        node.qhi_y[slot] = qh[1];
+        node.qhi_z[slot] = qh[2];
+        if (inner) {
+            next[levelOff + rank] = make_int2(x, childBase + rank);
+        } else if (isChild) {
+            // the leaf's triangles (code-order positions), left subtree first
+            int prim[kLeafMax] = {x, x, x};
+            if (leafTris > 1) {
+                const int2 cc = A.child[x];
+                if (leafTris == 2) {
+                    prim[0] = cc.x;
+                    prim[1] = cc.y;
+                } else if (cc.x >= A.n - 1) {
+                    const int2 c2 = A.child[cc.y];
+                    prim[0] = cc.x;
+                    prim[1] = c2.x;
+                    prim[2] = c2.y;
+                } else {
+                    const int2 c2 = A.child[cc.x];
+                    prim[0] = c2.x;
+                    prim[1] = c2.y;
+                    prim[2] = cc.y;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kLeafMax; q++) {
+                if (q >= leafTris) break;
+                const uint32_t id = A.order[prim[q] - (A.n - 1)];
+                const float *v = A.verts + 9 * static_cast<int64_t>(id);
                 TriRecord r;
-                r.v0 = make_float4(v[0], v[1], v[2], __int_as_float(static_cast<int>(prim)));
+                r.v0 = make_float4(v[0], v[1], v[2], __int_as_float(static_cast<int>(id)));
                 r.v1 = make_float4(v[3], v[4], v[5], 0.0f);
                 r.v2 = make_float4(v[6], v[7], v[8], 0.0f);
                 A.tris[triBase + triOff + q] = r;
                 A.slot_shade[triBase + triOff + q] =
-                    make_int2(A.tri_mat ? A.tri_mat[prim] : 0, A.tri_light ? A.tri_light[prim] : -1);
+                    make_int2(A.tri_mat ? A.tri_mat[id] : 0, A.tri_light ? A.tri_light[id] : -1);
             }
-            triOff += count;
         }
     }
-    A.nodes[w] = node;
 }
 
 template <class T>
@@ -498,6 +761,18 @@ T *dalloc(size_t n) {
     if (cudaMalloc(&p, sizeof(T) * std::max<size_t>(n, 1)) != cudaSuccess) return nullptr;
     return p;
 }
+
+// hands out 256-byte aligned pieces of one allocation; with base null it only adds them up
+struct Scratch {
+    unsigned char *base = nullptr;
+    size_t used = 0;
+    template <class T>
+    T *take(size_t n) {
+        const size_t at = used;
+        used = (used + sizeof(T) * std::max<size_t>(n, 1) + 255) & ~size_t(255);
+        return base ? reinterpret_cast<T *>(base + at) : nullptr;
+    }
+};
 
 }  // namespace
 
@@ -515,35 +790,59 @@ int buildWideBVH(const float *d_verts, int n, const int *d_tri_mat, const int *d
         snprintf(err, errlen, "buildWideBVH: empty scene");
         return -2;
     }
-    const int nNodes = 2 * n - 1;
-    float *d_bounds = dalloc<float>(12);
-    uint64_t *keys[2] = {dalloc<uint64_t>(n), dalloc<uint64_t>(n)};
-    uint32_t *vals[2] = {dalloc<uint32_t>(n), dalloc<uint32_t>(n)};
-    int2 *child = dalloc<int2>(n);
-    int *count = dalloc<int>(nNodes);
-    int *clusters[2] = {dalloc<int>(n), dalloc<int>(n)};
-    int *nn = dalloc<int>(n), *lead = dalloc<int>(n), *keep = dalloc<int>(n);
-    int *leadOff = dalloc<int>(n), *keepOff = dalloc<int>(n);
-    float4 *bmin = dalloc<float4>(nNodes);
-    float4 *bmax = dalloc<float4>(nNodes);
-    DpArgs dp{dalloc<float>(8 * static_cast<size_t>(nNodes)), dalloc<uint8_t>(8 * static_cast<size_t>(nNodes)),
-              dalloc<uint8_t>(n), dalloc<uint8_t>(nNodes)};
-    int2 *items[2] = {dalloc<int2>(n), dalloc<int2>(n)};
-    int *counters = dalloc<int>(4);
-    out->nodes = dalloc<WideNode>(n);
-    out->tris = dalloc<TriRecord>(n);
-    out->slot_shade = dalloc<int2>(n);
     int rc = 0;
-    void *tmp = nullptr, *scanTmp = nullptr;
-    size_t tmpBytes = 0, scanBytes = 0;
     auto fail = [&](const char *what, cudaError_t e) {
         snprintf(err, errlen, "buildWideBVH: %s: %s", what, cudaGetErrorString(e));
         rc = -3;
     };
-    if (!d_bounds || !keys[0] || !keys[1] || !vals[0] || !vals[1] || !child || !count || !clusters[0] ||
-        !clusters[1] || !nn || !lead || !keep || !leadOff || !keepOff || !bmin || !bmax || !dp.cost || !dp.split ||
-        !dp.wideSplit || !dp.leaf || !items[0] || !items[1] ||
-        !counters || !out->nodes || !out->tris || !out->slot_shade) {
+    const size_t N = static_cast<size_t>(n), nNodes = 2 * N - 1;
+    constexpr int kMaxLevels = 4096 / 64;   // more than the traversal accepts (kStackDepth)
+    static_assert(kMaxLevels > kStackDepth, "the depth check needs the levels past the limit");
+    float *d_bounds = nullptr;
+    uint64_t *keys[2] = {};
+    uint32_t *vals[2] = {};
+    int2 *child = nullptr, *items[2] = {};
+    int *count = nullptr, *clusters[2] = {}, *nn = nullptr;
+    uint32_t *sums = nullptr;
+    float4 *bmin = nullptr, *bmax = nullptr;
+    DpArgs dp{};
+    RoundState *rounds = nullptr;
+    unsigned long long *level = nullptr;
+    void *tmp = nullptr;
+    size_t tmpBytes = 0;
+    {
+        cub::DoubleBuffer<uint64_t> kb(keys[0], keys[1]);
+        cub::DoubleBuffer<uint32_t> vb(vals[0], vals[1]);
+        cub::DeviceRadixSort::SortPairs(nullptr, tmpBytes, kb, vb, n, 0, 64, stream);
+    }
+    // all scratch in one allocation: sized, then handed out
+    Scratch sc;
+    for (int pass = 0; pass < 2; pass++) {
+        sc.used = 0;
+        d_bounds = sc.take<float>(12);
+        for (int k = 0; k < 2; k++) {
+            keys[k] = sc.take<uint64_t>(N);
+            vals[k] = sc.take<uint32_t>(N);
+            clusters[k] = sc.take<int>(N);
+            items[k] = sc.take<int2>(N);
+        }
+        child = sc.take<int2>(N);
+        count = sc.take<int>(nNodes);
+        nn = sc.take<int>(N);
+        sums = sc.take<uint32_t>(N / kMergeBlock + 1);
+        bmin = sc.take<float4>(nNodes);
+        bmax = sc.take<float4>(nNodes);
+        dp = DpArgs{sc.take<float>(8 * N), sc.take<uint8_t>(8 * N), sc.take<uint8_t>(N), sc.take<uint8_t>(N)};
+        rounds = sc.take<RoundState>(kMaxRounds + 2);
+        level = sc.take<unsigned long long>(kMaxLevels + 1);
+        tmp = sc.take<unsigned char>(tmpBytes);
+        if (pass == 0 && cudaMalloc(&sc.base, sc.used) != cudaSuccess) break;
+    }
+    out->nodes = dalloc<WideNode>(n);
+    out->tris = dalloc<TriRecord>(n);
+    out->slot_shade = dalloc<int2>(n);
+    if (!sc.base || !out->nodes || !out->tris || !out->slot_shade) {
+        cudaGetLastError();
         snprintf(err, errlen, "buildWideBVH: device allocation failed for %d triangles", n);
         rc = -4;
     }
@@ -551,137 +850,107 @@ int buildWideBVH(const float *d_verts, int n, const int *d_tri_mat, const int *d
         const float init[12] = {3e38f, 3e38f, 3e38f, -3e38f, -3e38f, -3e38f,
                                 3e38f, 3e38f, 3e38f, -3e38f, -3e38f, -3e38f};
         cudaMemcpyAsync(d_bounds, init, sizeof(init), cudaMemcpyHostToDevice, stream);
-        cudaMemsetAsync(counters, 0, sizeof(int) * 4, stream);
+        cudaMemsetAsync(level, 0, sizeof(unsigned long long) * (kMaxLevels + 1), stream);
         const int T = 256;
-        k_prim_bounds<<<std::min((n + T - 1) / T, 1216), T, 0, stream>>>(d_verts, n, d_bounds);
+        k_prim_bounds<<<std::min((n + kBoundsBlock - 1) / kBoundsBlock, 1216), kBoundsBlock, 0, stream>>>(d_verts, n,
+                                                                                                      d_bounds);
         k_morton<<<(n + T - 1) / T, T, 0, stream>>>(d_verts, n, d_bounds, keys[0], vals[0]);
         cub::DoubleBuffer<uint64_t> kb(keys[0], keys[1]);
         cub::DoubleBuffer<uint32_t> vb(vals[0], vals[1]);
-        cub::DeviceRadixSort::SortPairs(nullptr, tmpBytes, kb, vb, n, 0, 64, stream);
-        cub::DeviceScan::ExclusiveSum(nullptr, scanBytes, lead, leadOff, n, stream);
-        if (cudaMalloc(&tmp, tmpBytes) != cudaSuccess || cudaMalloc(&scanTmp, scanBytes) != cudaSuccess) {
-            snprintf(err, errlen, "buildWideBVH: sort scratch allocation failed");
-            rc = -4;
-        } else {
-            cub::DeviceRadixSort::SortPairs(tmp, tmpBytes, kb, vb, n, 0, 64, stream);
-            const uint64_t *sk = kb.Current();
-            const uint32_t *order = vb.Current();
-            (void)sk;
-            k_leaf_bounds<<<(n + T - 1) / T, T, 0, stream>>>(d_verts, order, n, bmin, bmax, count, clusters[0],
-                                                                 dp);
-            // clustering rounds: m clusters, merged nodes numbered downwards from top
-            int m = n, top = n - 2, cl = 0, rounds = 0;
-            std::vector<int2> roundIds;   // node ids created by each round, in round order
-            while (m > 1 && rc == 0) {
-                const int B = (m + kPlocBlock - 1) / kPlocBlock;
-                k_ploc_nn<<<B, kPlocBlock, 0, stream>>>(clusters[cl], m, bmin, bmax, nn);
-                k_ploc_flags<<<B, kPlocBlock, 0, stream>>>(nn, m, lead, keep);
-                cub::DeviceScan::ExclusiveSum(scanTmp, scanBytes, lead, leadOff, m, stream);
-                cub::DeviceScan::ExclusiveSum(scanTmp, scanBytes, keep, keepOff, m, stream);
-                k_ploc_merge<<<B, kPlocBlock, 0, stream>>>(clusters[cl], m, nn, lead, leadOff, keep, keepOff, top,
-                                                           child, bmin, bmax, count, clusters[cl ^ 1]);
-                int tail[4] = {0, 0, 0, 0};   // leadOff, lead, keepOff, keep of the last cluster
-                cudaMemcpyAsync(&tail[0], leadOff + m - 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
-                cudaMemcpyAsync(&tail[1], lead + m - 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
-                cudaMemcpyAsync(&tail[2], keepOff + m - 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
-                cudaMemcpyAsync(&tail[3], keep + m - 1, sizeof(int), cudaMemcpyDeviceToHost, stream);
-                const cudaError_t e = cudaStreamSynchronize(stream);
-                if (e != cudaSuccess) {
-                    fail("clustering", e);
-                    break;
-                }
-                const int merges = tail[0] + tail[1];
-                if (merges > 0) roundIds.push_back(make_int2(top - merges + 1, top));
-                top -= merges;
-                m = tail[2] + tail[3];
-                cl ^= 1;
-                if (merges == 0 || ++rounds > 100000) {
-                    snprintf(err, errlen, "buildWideBVH: clustering made no progress");
-                    rc = -5;
-                }
-            }
-            if (rc == 0 && n > 1 && top != -1) {
-                snprintf(err, errlen, "buildWideBVH: clustering left %d node ids unused", top + 1);
+        cub::DeviceRadixSort::SortPairs(tmp, tmpBytes, kb, vb, n, 0, 64, stream);
+        const uint32_t *order = vb.Current();
+        k_leaf_bounds<<<(n + T - 1) / T, T, 0, stream>>>(d_verts, order, n, bmin, bmax, count, clusters[0]);
+        // clustering rounds (merged nodes numbered downwards), then the rest in one block
+        RoundState st{n, n - 2};
+        cudaError_t e = cudaMemcpyAsync(rounds, &st, sizeof(st), cudaMemcpyHostToDevice, stream);
+        int r = 0;
+        while (st.m > kTailClusters && e == cudaSuccess) {
+            if (r + kRoundsAhead > kMaxRounds) {
+                snprintf(err, errlen, "buildWideBVH: clustering made no progress");
                 rc = -5;
+                break;
             }
-            // the SAH programme, one launch per clustering round (children before parents)
-            for (const int2 r : roundIds) {
-                const int cnt = r.y - r.x + 1;
-                k_dp_round<<<(cnt + T - 1) / T, T, 0, stream>>>(child, count, bmin, bmax, r.x, r.y, dp, kLeafMax);
+            for (int k = 0; k < kRoundsAhead; k++, r++) {
+                const int *in = clusters[r & 1];
+                k_ploc_nn<<<(st.m + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, stream>>>(in, rounds + r, bmin, bmax, nn);
+                k_ploc_count<<<(st.m + kMergeBlock - 1) / kMergeBlock, kMergeBlock, 0, stream>>>(nn, rounds + r, sums);
+                k_ploc_merge<<<(st.m + kMergeBlock - 1) / kMergeBlock, kMergeBlock, 0, stream>>>(
+                    in, rounds + r, nn, sums, child, bmin, bmax, count, clusters[(r & 1) ^ 1]);
+                k_dp_round<<<(st.m / 2 + T - 1) / T, T, 0, stream>>>(child, count, bmin, bmax, rounds + r, n, dp);
             }
-            CollapseArgs A{d_verts, order, d_tri_mat, d_tri_light, n, child, count, dp, bmin, bmax,
-                           out->nodes, out->tris, out->slot_shade, counters};
-            // root: wide node 0 from binary root (internal 0, or the single leaf)
-            const int one = 1;
-            const int2 root = make_int2(n > 1 ? 0 : 0 + (n - 1), 0);
-            cudaMemcpyAsync(items[0], &root, sizeof(int2), cudaMemcpyHostToDevice, stream);
-            cudaMemcpyAsync(counters, &one, sizeof(int), cudaMemcpyHostToDevice, stream);
-            int nitems = rc == 0 ? 1 : 0, depth = 0, cur = 0;
-            while (nitems > 0) {
-                cudaMemsetAsync(counters + 2, 0, sizeof(int), stream);
-                k_collapse<<<(nitems + 127) / 128, 128, 0, stream>>>(A, items[cur], nitems, items[cur ^ 1]);
-                cudaMemcpyAsync(&nitems, counters + 2, sizeof(int), cudaMemcpyDeviceToHost, stream);
-                cudaError_t e = cudaStreamSynchronize(stream);
-                if (e != cudaSuccess) {
-                    fail("collapse", e);
-                    break;
-                }
-                cur ^= 1;
-                depth++;
-                if (depth > 4096) {
-                    snprintf(err, errlen, "buildWideBVH: collapse did not terminate");
-                    rc = -5;
-                    break;
-                }
+            const int before = st.m;
+            e = cudaMemcpyAsync(&st, rounds + r, sizeof(st), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (e == cudaSuccess && st.m >= before) {
+                snprintf(err, errlen, "buildWideBVH: clustering made no progress");
+                rc = -5;
+                break;
             }
-            int hostCounters[4] = {0, 0, 0, 0};
-            cudaMemcpyAsync(hostCounters, counters, sizeof(hostCounters), cudaMemcpyDeviceToHost, stream);
-            cudaError_t e = cudaStreamSynchronize(stream);
-            if (e != cudaSuccess && rc == 0) fail("final sync", e);
-            if (rc == 0) {
-                float hb[12];
-                cudaMemcpy(hb, d_bounds, sizeof(hb), cudaMemcpyDeviceToHost);
-                out->lo = mk(hb[0], hb[1], hb[2]);
-                out->hi = mk(hb[3], hb[4], hb[5]);
-                out->n_nodes = hostCounters[0];
-                out->ntri = n;
-                out->depth = depth;
-                if (hostCounters[1] != n) {
-                    snprintf(err, errlen, "buildWideBVH: placed %d of %d triangles", hostCounters[1], n);
-                    rc = -6;
-                } else if (depth > kStackDepth) {
-                    snprintf(err, errlen, "buildWideBVH: tree depth %d exceeds the traversal stack (%d)", depth,
-                             kStackDepth);
-                    rc = -7;
-                }
+        }
+        if (e == cudaSuccess && rc == 0) {
+            e = cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
+            if (e == cudaSuccess)
+                k_ploc_tail<<<1, kMergeBlock, kTailSmem, stream>>>(clusters[r & 1], rounds + r, child, bmin, bmax,
+                                                                   count, n, dp);
+        }
+        // the wide tree, kRoundsAhead levels between two looks at what they allocated
+        const int2 root = make_int2(n > 1 ? 0 : n - 1, 0);
+        cudaMemcpyAsync(items[0], &root, sizeof(int2), cudaMemcpyHostToDevice, stream);
+        CollapseArgs A{d_verts, order, d_tri_mat, d_tri_light, n, child, count, dp, bmin, bmax,
+                       out->nodes, out->tris, out->slot_shade, level};
+        unsigned long long got[kMaxLevels + 1] = {};
+        RoundState left{0, 0};
+        float hb[12] = {};
+        int depth = 0;
+        bool open = rc == 0;
+        while (open && e == cudaSuccess) {
+            long long most = 1;   // nodes of the first level launched now, at most eight times that in the next
+            if (depth > 0) most = static_cast<long long>(got[depth - 1] & 0xFFFFFFFFull);
+            for (int k = 0; k < kRoundsAhead && depth + k < kMaxLevels; k++) {
+                const long long blocks = (std::min<long long>(most, n) + kCollapseNodes - 1) / kCollapseNodes;
+                k_collapse<<<static_cast<int>(std::min<long long>(blocks, 152 * 16)), kCollapseBlock, 0, stream>>>(
+                    A, depth + k, items[(depth + k) & 1], items[((depth + k) & 1) ^ 1]);
+                most = std::min<long long>(8 * most, n);
+            }
+            e = cudaMemcpyAsync(got, level, sizeof(got), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess && depth == 0)
+                e = cudaMemcpyAsync(&left, rounds + r + 1, sizeof(left), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess && depth == 0) e = cudaMemcpyAsync(hb, d_bounds, sizeof(hb), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) break;
+            if (n > 1 && (left.m != 1 || left.top != -1)) {
+                snprintf(err, errlen, "buildWideBVH: clustering left %d clusters and %d node ids", left.m, left.top + 1);
+                rc = -5;
+                break;
+            }
+            for (int k = 0; k < kRoundsAhead && open && depth < kMaxLevels; k++) {
+                depth++;   // a level of at least one item has run
+                open = (got[depth - 1] & 0xFFFFFFFFull) != 0;
+            }
+            if (depth >= kMaxLevels) open = false;
+        }
+        if (e != cudaSuccess && rc == 0) fail("build", e);
+        if (rc == 0) {
+            long long nodes = 1, tris = 0;
+            for (int k = 0; k < depth; k++) {
+                nodes += static_cast<long long>(got[k] & 0xFFFFFFFFull);
+                tris += static_cast<long long>(got[k] >> 32);
+            }
+            out->lo = mk(hb[0], hb[1], hb[2]);
+            out->hi = mk(hb[3], hb[4], hb[5]);
+            out->n_nodes = static_cast<int>(nodes);
+            out->ntri = n;
+            out->depth = depth;
+            if (depth > kStackDepth) {
+                snprintf(err, errlen, "buildWideBVH: tree depth %d exceeds the traversal stack (%d)", depth, kStackDepth);
+                rc = -7;
+            } else if (tris != n) {
+                snprintf(err, errlen, "buildWideBVH: placed %lld of %d triangles", tris, n);
+                rc = -6;
             }
         }
     }
-    cudaFree(tmp);
-    cudaFree(scanTmp);
-    cudaFree(d_bounds);
-    cudaFree(keys[0]);
-    cudaFree(keys[1]);
-    cudaFree(vals[0]);
-    cudaFree(vals[1]);
-    cudaFree(child);
-    cudaFree(count);
-    cudaFree(clusters[0]);
-    cudaFree(clusters[1]);
-    cudaFree(nn);
-    cudaFree(lead);
-    cudaFree(keep);
-    cudaFree(leadOff);
-    cudaFree(keepOff);
-    cudaFree(bmin);
-    cudaFree(bmax);
-    cudaFree(dp.cost);
-    cudaFree(dp.split);
-    cudaFree(dp.wideSplit);
-    cudaFree(dp.leaf);
-    cudaFree(items[0]);
-    cudaFree(items[1]);
-    cudaFree(counters);
+    cudaFree(sc.base);
     if (rc != 0) freeWideBVH(out);
     return rc;
 }

@@ -75,3 +75,32 @@ def test_one_pass_render_matches_pass_by_pass(gpulib, room, width, height, spp, 
     x, y = a[..., :3], b[..., :3]
     close = (x - y).abs() <= 1e-5 * y.abs() + 1e-6 * float(y.abs().max())
     assert close.float().mean() > 0.999
+
+
+@pytest.mark.parametrize("triangles", [1, 2, 3, 4, 5, 31, 32, 33, 65, 1023, 1025, 2047, 2048, 2049, 2050, 5000, 20000])
+def test_build_sizes(gpulib, port, triangles):
+    """Trees on both sides of the build's steps (one block for the last 2048 clusters, rounds of
+    1024-cluster blocks before): every triangle is placed, and the closest hits of random rays
+    are the oracle's under the parity rules of tests/parity.py."""
+    import numpy as np
+    from parity import classify_closest
+    rng = np.random.default_rng(triangles)
+    c = rng.random((triangles, 1, 3)) * 2 - 1
+    size = np.where(rng.random((triangles, 1, 1)) < 0.02, 1.0, 1.5 / np.sqrt(triangles))
+    sc = scenes.Scene(verts=(c + size * (rng.random((triangles, 3, 3)) - 0.5)).reshape(-1, 9).astype(np.float32),
+                      tri_mat=np.zeros(triangles, np.int32), materials=np.array([scenes.lambert(0.5, 0.5, 0.5)]))
+    acc = GpuBVHAccel(sc).construct()
+    info = acc.info()
+    assert info.triangles == triangles and 1 <= info.wide_nodes <= max(1, triangles - 1) and info.depth >= 1
+    lo, hi = acc.worldBound()
+    v = sc.verts.reshape(-1, 3)
+    np.testing.assert_array_equal(np.array([lo, hi], np.float32), [v.min(0), v.max(0)])
+    target = sc.verts.reshape(-1, 3, 3)[rng.integers(0, triangles, 4000)].mean(1)
+    org = (2.5 * rng.normal(size=(4000, 3))).astype(np.float32)
+    d = target - org
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    prim, t, _, _ = acc.intersect(org, d)
+    pr, tr = port.scene(sc).trace(org.astype(np.float64), d.astype(np.float64))
+    r = classify_closest(sc.verts, org, d, prim, t, pr, tr)
+    assert r["fail"] == 0 and r["t_fail"] == 0, r
+    assert (prim >= 0).mean() > 0.9
