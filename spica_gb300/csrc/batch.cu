@@ -54,6 +54,7 @@ struct BatchState {
     int engine = SPGPU_BATCH_STREAM;
     StreamBatch *sb = nullptr;
     int poolSlots = 0, poolLanes = 0, iterations = 0;
+    int classMask = 0;   // the shading classes of the batch's materials
 };
 
 namespace {
@@ -278,6 +279,7 @@ int batchPrepare(spgpu_ctx *self, BatchState **slot, int count, const spgpu_batc
         rc = spgpu_upload_scene(self, it.ntri, it.verts, it.tri_mat, it.nmat, it.materials, it.tri_emit, 0, 0, nullptr);
         if (rc == 0) rc = spgpu_build_bvh(self);
         if (rc) break;
+        B->classMask |= C.classMask;
         const int nb = C.bvh.n_nodes, nt = C.bvh.ntri;
         std::vector<WideNode> hn(nb);
         std::vector<TriRecord> ht(nt);
@@ -385,7 +387,7 @@ int batchPrepare(spgpu_ctx *self, BatchState **slot, int count, const spgpu_batc
             float msBest = 3.0e38f;
             if (c.engine == SPGPU_BATCH_STREAM) {
                 StreamBatch *tb = nullptr;
-                rc = streamBatchCreate(C, &tb, merged, reduced, c.slots, c.lanes, kIters);
+                rc = streamBatchCreate(C, &tb, merged, reduced, B->classMask, c.slots, c.lanes, kIters);
                 std::vector<double> rms(reduced.size());
                 unsigned long long st[4];
                 for (int rep = 0; rep < 2 && rc == 0; rep++) {
@@ -445,7 +447,7 @@ int batchPrepare(spgpu_ctx *self, BatchState **slot, int count, const spgpu_batc
             tuning->calib_ms = calibMs;
         }
         if (rc == 0 && B->engine == SPGPU_BATCH_STREAM) {
-            rc = streamBatchCreate(C, &B->sb, merged, B->hostMeta, B->poolSlots, B->poolLanes, B->iterations);
+            rc = streamBatchCreate(C, &B->sb, merged, B->hostMeta, B->classMask, B->poolSlots, B->poolLanes, B->iterations);
         } else if (rc == 0) {
             std::vector<BatchItem> its;
             std::vector<int> per;

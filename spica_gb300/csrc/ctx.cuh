@@ -243,8 +243,9 @@ struct RenderMeta {
 // iteration loop runs on the device (a CUDA graph with a conditional while node), so a
 // run is one graph launch
 struct StreamBatch;
+// (classMask: the shading classes of the batch's materials)
 int streamBatchCreate(Ctx &C, StreamBatch **slot, const SceneView &merged, const std::vector<RenderMeta> &renders,
-                      int poolSlots, int lanes, int iterations);
+                      int classMask, int poolSlots, int lanes, int iterations);
 int streamBatchRun(Ctx &C, StreamBatch &SB, float4 *film, double *renderMs, unsigned long long *statsOut,
                    float *msOut, cudaStream_t stream);
 int streamBatchProfile(Ctx &C, StreamBatch &SB, float4 *film, double *kernelMs, long long *launches,

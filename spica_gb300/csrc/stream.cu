@@ -110,6 +110,15 @@ struct StreamArgs {
     float4 *rO, *rD, *rB;
     // class queues, cap rows per class: the pool record and the hit (t, slot, u, v)
     float4 *qO, *qD, *qB, *qH;
+    // Where continuations go: the pool itself, or, in scenes of one shading class (singleClass,
+    // else -1), the other of two pools, rays and continuations changing places every iteration.
+    // There the class queue would only copy the pool: extend leaves the hit of pool ray i in
+    // qH[i] (slot -1: none) and the class's shading reads the pool.  The second pool is the
+    // space of the class queues, which such scenes do not use.  A vertex then moves 96 bytes
+    // less and its extend appends to no queue: a batch of 16 box rooms 150.1 -> 146.4 ms, the
+    // guided room at 640 x 360 3.30 -> 3.16.
+    float4 *nO, *nD, *nB;
+    int singleClass;
     float4 *shO, *shD, *shL;   // shadow queue, 2 * cap rows: (origin, film index), (dir, tmax), contribution
     int *ctr;
     int *cont;         // continuations written
@@ -241,7 +250,7 @@ __global__ void k_sregen(StreamArgs p) {
 
 // closest hit of the pool's rays into the class queues (every thread of the block)
 // (OWN other than kFromCounter: a one-pass render, whose counter holds all its rays)
-template <bool STATS, bool BATCH, bool SPLIT, int OWN = kFromCounter>
+template <bool STATS, bool BATCH, bool SPLIT, bool SINGLE, int OWN = kFromCounter>
 __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
     uint32_t nodeCount = 0, triCount = 0;
     const int n = p.ctr[kCtrRays] + (OWN != kFromCounter ? 0 : newPaths(p));
@@ -249,6 +258,22 @@ __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
     bool overflow = false;
     auto done = [&](int i, const TraceLane &L) {
         if (!__any_sync(0xffffffffu, i >= 0)) return;
+        if constexpr (SINGLE) {
+            int render = 0;
+            if (i >= 0) {
+                p.qH[i] = make_float4(L.tmax, __int_as_float(L.found ? L.hitSlot : -1), L.hu, L.hv);
+                if (!L.found && (BATCH || p.sv.hasEnv)) {
+                    const int meta = __float_as_int(p.rD[i].w);
+                    if (BATCH) render = metaRender(meta);
+                    else if ((meta & 255) == 0 || (meta & 256)) {
+                        const float3 c = xyz(p.rB[i]) * envLe(p.sv.env, L.d);
+                        atomicAdd(&film[filmIndexS(p, __float_as_int(p.rO[i].w))], make_float4(c.x, c.y, c.z, 0.0f));
+                    }
+                }
+            }
+            if constexpr (BATCH) countEnded(p, i >= 0 && !L.found, render);   // no environment
+            return;
+        }
         int cls = -1;
         float4 o4 = make_float4(0, 0, 0, 0), d4 = o4, b4 = o4;
         if (i >= 0) {
@@ -310,10 +335,10 @@ __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
     }
 }
 
-template <bool STATS, bool BATCH, bool SPLIT>
+template <bool STATS, bool BATCH, bool SPLIT, bool SINGLE>
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(StreamArgs p) {
     __shared__ uint2 stack[kStackShared * kTraceBlock];
-    extendQueue<STATS, BATCH, SPLIT>(p, stack);
+    extendQueue<STATS, BATCH, SPLIT, SINGLE>(p, stack);
 }
 
 // one shadow ray into the shadow queue; the lanes that have one at the same point of the
@@ -335,10 +360,25 @@ __device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const Shad
     if constexpr (BATCH) countEnded(p, live && !R.cont, metaRender(meta));
     const int k = warpAppendS(R.cont && !p.direct, p.cont);
     if (k >= 0) {
-        p.rO[k] = make_float4(R.cO.x, R.cO.y, R.cO.z, __int_as_float(pix));
-        p.rD[k] = make_float4(R.cD.x, R.cD.y, R.cD.z, packMeta((meta & 255) + 1, R.spec, metaRender(meta)));
-        p.rB[k] = make_float4(R.beta.x, R.beta.y, R.beta.z, __int_as_float(sample));
+        p.nO[k] = make_float4(R.cO.x, R.cO.y, R.cO.z, __int_as_float(pix));
+        p.nD[k] = make_float4(R.cD.x, R.cD.y, R.cD.z, packMeta((meta & 255) + 1, R.spec, metaRender(meta)));
+        p.nB[k] = make_float4(R.beta.x, R.beta.y, R.beta.z, __int_as_float(sample));
     }
+}
+
+// the rows that class cls shades in this iteration: its queue, or the pool's rays where the
+// scene has that class alone
+struct ShadeRows {
+    const float4 *o, *d, *b, *h;
+    int n;
+};
+__device__ __forceinline__ ShadeRows shadeRows(const StreamArgs &p, int cls) {
+    if (p.singleClass >= 0) {
+        const int rays = p.ctr[kCtrRays] + (p.onePass ? 0 : newPaths(p));
+        return {p.rO, p.rD, p.rB, p.qH, p.singleClass == cls ? rays : 0};
+    }
+    const int64_t base = static_cast<int64_t>(cls) * p.cap;
+    return {p.qO + base, p.qD + base, p.qB + base, p.qH + base, p.ctr[kCtrClass0 + cls]};
 }
 
 __device__ __forceinline__ HitRecord hitOfRow(float4 h4) {
@@ -361,18 +401,24 @@ __device__ __forceinline__ HitRecord hitOfRow(float4 h4) {
 template <int CLS, bool BATCH>
 __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(StreamArgs p) {
     awaitLastKernel();
-    const int n = p.ctr[kCtrClass0 + CLS];
+    const ShadeRows rows = shadeRows(p, CLS);
+    const int n = rows.n;
     const int stride = gridDim.x * blockDim.x;
     const int nIter = (n + stride - 1) / stride;   // uniform trip count keeps warps whole for the ballots
-    const int64_t base = static_cast<int64_t>(CLS) * p.cap;
     for (int it = 0; it < nIter; it++) {
         const int j = it * stride + blockIdx.x * blockDim.x + threadIdx.x;
         ShadeOut R;
         R.cont = false;
         int pix = 0, meta = 0, sample = 0;
         long long filmIdx = 0;
+        bool live = false;
+        float4 h4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (j < n) {
-            const float4 o4 = p.qO[base + j], d4 = p.qD[base + j], b4 = p.qB[base + j], h4 = p.qH[base + j];
+            h4 = rows.h[j];
+            live = p.singleClass < 0 || __float_as_int(h4.y) >= 0;   // a class queue holds hits only
+        }
+        if (live) {
+            const float4 o4 = rows.o[j], d4 = rows.d[j], b4 = rows.b[j];
             pix = __float_as_int(o4.w);
             meta = __float_as_int(d4.w);
             sample = __float_as_int(b4.w);
@@ -400,7 +446,7 @@ __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(St
                                 p.direct != 0, [&](int, float4 so, float4 sd, float4 sl) { appendShadow(p, so, sd, sl); });
             }
         }
-        emitShadeResultS<BATCH>(p, R, j < n, filmIdx, pix, meta, sample);
+        emitShadeResultS<BATCH>(p, R, live, filmIdx, pix, meta, sample);
     }
 }
 
@@ -413,10 +459,10 @@ __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(St
 // launch per bounce.
 __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(StreamArgs p) {
     awaitLastKernel();
-    const int n = p.ctr[kCtrClass0 + kMatLambert];
+    const ShadeRows rows = shadeRows(p, kMatLambert);
+    const int n = rows.n;
     if (static_cast<int>(blockIdx.x) * kGTile >= n) return;   // no tile for this CTA
     extern __shared__ __align__(128) uint8_t sm[];
-    const int64_t base = static_cast<int64_t>(kMatLambert) * p.cap;
     bool ok = true;
     const uint32_t tmem = tileKernelSetup(sm, p.packFwd, p.biasPad, &ok, kGsOffBar);
     const float *bias = reinterpret_cast<const float *>(sm + kTileSmOffBias);
@@ -426,16 +472,19 @@ __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(Stre
     uint32_t phase = 0;
     for (int tile = blockIdx.x; ok && tile * kGTile < n; tile += gridDim.x) {
         const int j = tile * kGTile + static_cast<int>(threadIdx.x);
-        const bool live = j < n;
-        float4 o4 = make_float4(0, 0, 0, 0), d4 = make_float4(0, 0, 1, 0), b4 = o4, h4 = o4;
+        float4 o4 = make_float4(0, 0, 0, 0), d4 = make_float4(0, 0, 1, 0), b4 = o4;
+        float4 h4 = make_float4(0.0f, __int_as_float(-1), 0.0f, 0.0f);
+        if (j < n) {
+            o4 = rows.o[j];
+            d4 = rows.d[j];
+            b4 = rows.b[j];
+            h4 = rows.h[j];
+        }
+        const bool live = __float_as_int(h4.y) >= 0;
         float3 ps = mk(0, 0, 0), nn = mk(0, 0, 1);
         float xf[16];
         for (int k = 0; k < 16; k++) xf[k] = 0.0f;
         if (live) {
-            o4 = p.qO[base + j];
-            d4 = p.qD[base + j];
-            b4 = p.qB[base + j];
-            h4 = p.qH[base + j];
             ps = hitPoint(xyz(o4), xyz(d4), h4.x);
             nn = triNormal(p.sv.tris[__float_as_int(h4.y)]);
             guideFeatures(ps, nn, -xyz(d4), p.guideLo, p.guideInvExt, xf);
@@ -529,11 +578,11 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sshadow(Stream
 // One-pass renders: an iteration's closest hits (EXTEND) and the last iteration's shadow rays,
 // which do not depend on each other, in one launch; a warp that finds no more of the first
 // goes on with the second.
-template <bool EXTEND, bool SPLIT>
+template <bool EXTEND, bool SPLIT, bool SINGLE>
 __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_strace(StreamArgs p) {
     __shared__ uint2 stack[kStackShared * kTraceBlock];
     awaitLastKernel();
-    if constexpr (EXTEND) extendQueue<false, false, SPLIT, kOwnFromFirst>(p, stack);
+    if constexpr (EXTEND) extendQueue<false, false, SPLIT, SINGLE, kOwnFromFirst>(p, stack);
     if (p.shadowCtr) shadowQueue<false, false, SPLIT, kOwnFromLast>(p, p.shadowCtr, stack);
 }
 
@@ -579,13 +628,33 @@ struct GridsS {
     int trace, shade, regen, guided;
 };
 
+// The traversal kernels' eight blocks per SM use 64 KB of shared memory.  A carveout of a third
+// (72 of 228 KB) leaves the rest to L1, which serves half of their node loads: 30 / 40 / 60 % and
+// the driver's choice, a batch of 16 box rooms 145.2 / 145.1 / 148.1 / 146.3 ms, the mid-scale
+// render 25.51 / 25.53 / 25.72 / 25.62.  (Not for k_strace, whose launches alternate with small
+// shading launches.)
+bool preferL1() {
+    for (const void *k : {reinterpret_cast<const void *>(k_sextend<false, false, false, false>),
+                          reinterpret_cast<const void *>(k_sextend<false, false, false, true>),
+                          reinterpret_cast<const void *>(k_sextend<false, false, true, false>),
+                          reinterpret_cast<const void *>(k_sextend<false, false, true, true>),
+                          reinterpret_cast<const void *>(k_sextend<false, true, false, false>),
+                          reinterpret_cast<const void *>(k_sextend<false, true, false, true>),
+                          reinterpret_cast<const void *>(k_sshadow<false, false, false>),
+                          reinterpret_cast<const void *>(k_sshadow<false, false, true>),
+                          reinterpret_cast<const void *>(k_sshadow<false, true, false>)})
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 32);
+    cudaGetLastError();   // a preference
+    return true;
+}
+
 GridsS streamGrids(int device, int cap, bool guided) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     // resident blocks per SM: properties of the compiled kernels
     static const int occT = [] {
         int o = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sextend<false, false, true>, kTraceBlock, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sextend<false, false, true, false>, kTraceBlock, 0);
         return o;
     }();
     static const int occS = [] {
@@ -593,6 +662,8 @@ GridsS streamGrids(int device, int cap, bool guided) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k_sshade<0, false>, kShadeBlockS, 0);
         return o;
     }();
+    static const bool carved = preferL1();
+    (void)carved;
     GridsS g;
     g.trace = sms * std::max(occT, 1);
     g.shade = sms * std::max(occS, 1);
@@ -618,6 +689,24 @@ cudaError_t launchStreamKernel(K kernel, int grid, int block, size_t smem, cudaS
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
+// Pools and class of a render's iterations: two pools where the scene has one shading class (its
+// mask has one bit), the pool and the class queues otherwise.
+void setPools(StreamArgs &a, int classMask) {
+    a.singleClass = classMask == 1 ? 0 : classMask == 2 ? 1 : classMask == 4 ? 2 : -1;
+    a.nO = a.singleClass >= 0 ? a.qO : a.rO;
+    a.nD = a.singleClass >= 0 ? a.qD : a.rD;
+    a.nB = a.singleClass >= 0 ? a.qB : a.rB;
+}
+// every other iteration's arguments
+StreamArgs poolsSwapped(StreamArgs a) {
+    if (a.singleClass >= 0) {
+        std::swap(a.rO, a.nO);
+        std::swap(a.rD, a.nD);
+        std::swap(a.rB, a.nB);
+    }
+    return a;
+}
+
 // the shading kernels of the classes in mask; returns how many
 template <bool BATCH>
 int launchShading(const StreamArgs &a, const GridsS &g, cudaStream_t s, int mask) {
@@ -638,10 +727,11 @@ int launchShading(const StreamArgs &a, const GridsS &g, cudaStream_t s, int mask
     return n;
 }
 
-// one iteration on stream s; with ev, every kernel is bracketed by a pair of events
+// one iteration on stream s with the shading classes in mask; with ev, every kernel is bracketed
+// by a pair of events
 template <bool STATS, bool BATCH = false>
-void launchIteration(const StreamArgs &a, const GridsS &g, cudaStream_t s, cudaEvent_t *ev, int *evClass,
-                     int *nev) {
+void launchIteration(const StreamArgs &a, const GridsS &g, cudaStream_t s, cudaEvent_t *ev, int *evClass, int *nev,
+                     int mask = 7) {
     auto mark = [&](int cls) {
         if (ev) {
             evClass[*nev / 2] = cls;
@@ -657,10 +747,14 @@ void launchIteration(const StreamArgs &a, const GridsS &g, cudaStream_t s, cudaE
     k_sregen<BATCH><<<g.regen, 256, 0, s>>>(a);
     done();
     mark(kSExtend);
-    if (split) k_sextend<STATS, BATCH, !BATCH><<<g.trace, kTraceBlock, 0, s>>>(a);
-    else k_sextend<STATS, BATCH, false><<<g.trace, kTraceBlock, 0, s>>>(a);
+    const bool single = !STATS && a.singleClass >= 0;
+    if (split && single) k_sextend<STATS, BATCH, !BATCH, !STATS><<<g.trace, kTraceBlock, 0, s>>>(a);
+    else if (split) k_sextend<STATS, BATCH, !BATCH, false><<<g.trace, kTraceBlock, 0, s>>>(a);
+    else if (single) k_sextend<STATS, BATCH, false, !STATS><<<g.trace, kTraceBlock, 0, s>>>(a);
+    else k_sextend<STATS, BATCH, false, false><<<g.trace, kTraceBlock, 0, s>>>(a);
     done();
     for (int c = 0; c < 3; c++) {
+        if (!((mask >> c) & 1)) continue;
         mark(kSShadeL + c);
         launchShading<BATCH>(a, g, s, 1 << c);
         done();
@@ -749,6 +843,7 @@ int setupStream(Ctx &C, StreamQueues &q, const float *camera, int W, int H, int 
     a.ctr = q.ctr;
     a.cont = q.ctr + kCtrCont;
     a.big = q.big;
+    setPools(a, C.classMask);
     if (gv) {
         a.packFwd = gv->packFwd;
         a.biasPad = gv->biasPad;
@@ -772,7 +867,9 @@ int ensureStreamGraph(Ctx &C, StreamQueues &q, const StreamArgs &a, cudaStream_t
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cudaFail("cudaStreamBeginCapture", e);
-    for (int it = 0; it < kIterPerGraph; it++) launchIteration<false>(a, g, s, nullptr, nullptr, nullptr);
+    static_assert(kIterPerGraph % 2 == 0, "the two pools of a one-class scene end up in their places");
+    for (int it = 0; it < kIterPerGraph; it++)
+        launchIteration<false>(it % 2 ? poolsSwapped(a) : a, g, s, nullptr, nullptr, nullptr);
     e = cudaStreamEndCapture(s, &graph);
     if (e != cudaSuccess) return cudaFail("cudaStreamEndCapture", e);
     e = cudaGraphInstantiate(&q.graph, graph, 0);
@@ -824,6 +921,8 @@ __global__ void k_sbatch_reset(BatchReset in) {
 
 }  // namespace
 
+inline int popcount3(int mask) { return (mask & 1) + (mask >> 1 & 1) + (mask >> 2 & 1); }
+
 struct StreamBatch {
     int lanes = 1, iterations = 0;
     StreamQueues q[Ctx::kPoolLanes];   // the batch's own pools (the context's serve spgpu_render)
@@ -831,7 +930,7 @@ struct StreamBatch {
     RenderMeta *renders = nullptr;     // device
     long long *pathStart = nullptr;    // device, nRenders + 1
     unsigned long long *ended = nullptr, *times = nullptr;
-    int nRenders = 0, maxDepth = 0;
+    int nRenders = 0, maxDepth = 0, classMask = 7;
     std::vector<long long> hostStart;
     cudaGraphExec_t exec = nullptr;
     float4 *execFilm = nullptr;
@@ -849,7 +948,7 @@ void freeStreamBatch(StreamBatch *SB) {
 }
 
 int streamBatchCreate(Ctx &C, StreamBatch **slot, const SceneView &merged, const std::vector<RenderMeta> &renders,
-                      int poolSlots, int lanes, int iterations) {
+                      int classMask, int poolSlots, int lanes, int iterations) {
     freeStreamBatch(*slot);
     *slot = nullptr;
     // a path carries its render in bits 9..30 of its meta word
@@ -861,6 +960,7 @@ int streamBatchCreate(Ctx &C, StreamBatch **slot, const SceneView &merged, const
     auto *SB = new StreamBatch();
     SB->lanes = lanes;
     SB->iterations = iterations;
+    SB->classMask = classMask;
     SB->sv = merged;
     SB->nRenders = static_cast<int>(renders.size());
     SB->hostStart.assign(renders.size() + 1, 0);
@@ -915,6 +1015,8 @@ StreamArgs batchLaneArgs(const StreamBatch &SB, int k, cudaGraphConditionalHandl
     a.ctr = q.ctr;
     a.cont = q.ctr + kCtrCont;
     a.big = q.big;
+    // an odd number of iterations would leave the rays in the other pool
+    setPools(a, SB.iterations % 2 == 0 ? SB.classMask : 0);
     a.renders = SB.renders;
     a.pathStart = SB.pathStart;
     a.nRenders = SB.nRenders;
@@ -973,7 +1075,8 @@ int buildBatchGraph(Ctx &C, StreamBatch &SB, float4 *film) {
         a.iterLimit = iterationBound(a, init.count[k]);
         e = cudaStreamBeginCaptureToGraph(cs, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e != cudaSuccess) break;
-        for (int it = 0; it < SB.iterations; it++) launchIteration<false, true>(a, g, cs, nullptr, nullptr, nullptr);
+        for (int it = 0; it < SB.iterations; it++)
+            launchIteration<false, true>(it % 2 ? poolsSwapped(a) : a, g, cs, nullptr, nullptr, nullptr, SB.classMask);
         e = cudaStreamEndCapture(cs, &body);
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&SB.exec, G, 0);
@@ -1022,7 +1125,8 @@ int streamBatchRun(Ctx &C, StreamBatch &SB, float4 *film, double *renderMs, unsi
         statsOut[0] += big[k][kBigPaths];
         statsOut[1] += big[k][kBigClosest];
         statsOut[2] += big[k][kBigShadow];
-        statsOut[3] += big[k][kBigIters] * kSNumClasses + 1;
+        // an iteration: regen, extend, the batch's shading classes, shadow, advance; and the reset
+        statsOut[3] += big[k][kBigIters] * (4 + popcount3(SB.classMask)) + 1;
         err |= ctr[k][kCtrErr];
         drained = drained && ctr[k][kCtrDone];
     }
@@ -1135,8 +1239,11 @@ int renderOnePass(Ctx &C, const float *camera, int W, int H, int spp, int sample
             p.ctr = C.sq[k].ctr + kNumCtr * it;
             p.cont = p.ctr + kNumCtr + kCtrRays;
             p.shadowCtr = it > 0 ? p.ctr - kNumCtr : nullptr;
-            if (split) launchStreamKernel(k_strace<true, true>, g.trace, kTraceBlock, 0, ls[k], p);
-            else launchStreamKernel(k_strace<true, false>, g.trace, kTraceBlock, 0, ls[k], p);
+            if (it > 0) p = poolsSwapped(p);
+            const bool single = p.singleClass >= 0;
+            launchStreamKernel(split ? (single ? k_strace<true, true, true> : k_strace<true, true, false>)
+                                     : (single ? k_strace<true, false, true> : k_strace<true, false, false>),
+                               g.trace, kTraceBlock, 0, ls[k], p);
             launches++;
             launches += launchShading<false>(p, g, ls[k], C.classMask);
             e = cudaGetLastError();
@@ -1145,8 +1252,8 @@ int renderOnePass(Ctx &C, const float *camera, int W, int H, int spp, int sample
     if (direct || done < iters) {   // the shadow rays of the last iteration launched
         for (int k = 0; k < lanes && e == cudaSuccess; k++) {
             a[k].shadowCtr = C.sq[k].ctr + kNumCtr * (done - 1);
-            if (split) launchStreamKernel(k_strace<false, true>, g.trace, kTraceBlock, 0, ls[k], a[k]);
-            else launchStreamKernel(k_strace<false, false>, g.trace, kTraceBlock, 0, ls[k], a[k]);
+            launchStreamKernel(split ? k_strace<false, true, false> : k_strace<false, false, false>, g.trace, kTraceBlock, 0,
+                               ls[k], a[k]);
             launches++;
             e = cudaGetLastError();
         }
@@ -1315,6 +1422,7 @@ int renderStreamProfile(Ctx *ctx, const float *camera, int W, int H, int spp, in
     StreamArgs a;
     StreamQueues &q = C.sq[0];
     if (int rc = setupStream(C, q, camera, W, H, spp, maxDepth, seed, integrator, gv, &a)) return rc;
+    setPools(a, 7);   // through the class queues, whose kernels the profile times
     const GridsS g = streamGrids(C.device, a.cap, a.packFwd != nullptr);
     const long long total = static_cast<long long>(W) * H * spp;
     const StreamInit init = streamInit(total, sampleOffset, film);
@@ -1377,6 +1485,7 @@ int streamBatchProfile(Ctx &C, StreamBatch &SB, float4 *film, double *kernelMs, 
     }
     for (int k = 0; k < 4; k++) statsOut[k] = visitOut[k] = 0;
     StreamArgs a = batchLaneArgs(SB, 0, 0);
+    setPools(a, 7);   // through the class queues, whose kernels the profile times
     const long long total = SB.hostStart.back();
     a.iterLimit = iterationBound(a, total);
     BatchReset init;

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(kShadeBlock) k_shade(PassArgs p, int b) {
             const float4 bt = p.beta[pid];
             const int fi = filmIndex(p, pid);
             // shadow rays carry the film pixel, or the path when collecting (k_shadow)
-            shadeHit<CLS>(p.sv, p.hits[i], xyz(o4), xyz(d4), xyz(bt), bt.w != 0.0f, b, p.maxDepth, p.seed,
+            shadeHit(p.sv, p.hits[i], xyz(o4), xyz(d4), xyz(bt), bt.w != 0.0f, b, p.maxDepth, p.seed,
                      static_cast<uint32_t>(fi), sample, p.collect ? pid : fi, R, p.direct != 0);
             if (!isBlack(R.emit)) {
                 if (p.collect) gather<true>(p, pid, fi, R.emit);

@@ -104,3 +104,40 @@ def test_build_sizes(gpulib, port, triangles):
     r = classify_closest(sc.verts, org, d, prim, t, pr, tr)
     assert r["fail"] == 0 and r["t_fail"] == 0, r
     assert (prim >= 0).mean() > 0.9
+
+
+def _one_class_room(cls, width, height):
+    sc = ROOMS["material" if cls == 2 else "box" if cls == 0 else "conductor"](width=width, height=height)
+    if cls == 1:      # rough conductors alone
+        sc.materials = sc.materials[-2:]
+        sc.tri_mat = (sc.tri_mat % 2).astype(sc.tri_mat.dtype)
+    elif cls == 2:    # plastic alone
+        sc.materials = sc.materials[-1:]
+        sc.tri_mat = 0 * sc.tri_mat
+    return sc
+
+
+@pytest.mark.parametrize("cls", [0, 1, 2])
+@pytest.mark.parametrize("width, height, spp", [(64, 48, 3), (3001, 3000, 2)])   # one pass; the refilling loop
+def test_one_class_scene_matches_pass_by_pass(gpulib, cls, width, height, spp):
+    """Scenes of one shading class are shaded out of the pool itself, rays and continuations in
+    two pools that change places; rays leave the rooms through their open side, so there are
+    rows without a hit.  Same samples and rays as the pass-by-pass wavefront, films equal up to
+    the order of their additions (the bounds of test_one_pass_render_matches_pass_by_pass)."""
+    import torch
+    from spica_gb300 import Context, GpuPathIntegrator
+    sc = _one_class_room(cls, width, height)
+    params = {"width": width, "height": height, "maxDepth": 5, "sampleCount": spp}
+    got = []
+    for wavefront in (0, 1):
+        acc = GpuBVHAccel(sc, ctx=Context(0, pass_lanes=1, wavefront=wavefront)).construct()
+        film = torch.zeros((height, width, 4), device="cuda")
+        st = GpuPathIntegrator(seed=8).render_device(sc.camera, acc, params, film)
+        got.append((film, st.paths, st.rays_closest, st.rays_shadow))
+        del acc
+    (a, *sa), (b, *sb) = got
+    assert sa == sb and sa[0] == width * height * spp
+    assert torch.equal(a[..., 3], b[..., 3])
+    x, y = a[..., :3], b[..., :3]
+    close = (x - y).abs() <= 1e-5 * y.abs() + 1e-6 * float(y.abs().max())
+    assert close.float().mean() > 0.999
