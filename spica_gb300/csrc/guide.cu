@@ -29,8 +29,7 @@ struct GuideState {
     int capacity = 0;
     int *ctl = nullptr;         // [0] samples written (monotonic), [1] error, [2] work counter
     double *lossAcc = nullptr;  // [0] loss sum, [1] weight sum
-    float *wsum = nullptr;      // batch weight sum / max
-    float *batch = nullptr;
+    float *wsum = nullptr;      // batch weight sums: of this step, the next and the last (kWsumSlots)
     int batchCap = 0;
     float *partials = nullptr;  // per training CTA: its partial gradient (kGParams floats)
     int partialRows = 0;
@@ -129,7 +128,6 @@ __device__ __forceinline__ float mixtureLossGrad(const float *r, float3 w, float
 }
 
 // ------------------------------------------------------------------ training
-constexpr int kTrainStride = 65;   // fp32 row stride of the dy tile
 struct TrainLayout {
     static constexpr int wf = 0;
     static constexpr int wb = wf + kPackFwdBytes;
@@ -139,9 +137,8 @@ struct TrainLayout {
     static constexpr int h2 = h1 + kGTile * kGHid * 2;
     static constexpr int h3 = h2 + kGTile * kGHid * 2;
     static constexpr int dyb = h3 + kGTile * kGHid * 2;
-    static constexpr int dy = dyb + kGTile * kGHid * 2;
-    static constexpr int gb = dy + kGTile * kTrainStride * 4;
-    static constexpr int bar = gb + kBiasPad * 4;
+    static constexpr int gb = dyb + kGTile * kGHid * 2;
+    static constexpr int bar = gb + kGTile / 32 * kBiasPad * 4;
     static constexpr int tmem = bar + 8;
     static constexpr int loadBar = tmem + 8;
     static constexpr int total = loadBar + 8;
@@ -174,13 +171,26 @@ __device__ __forceinline__ void issueWeightGrad(uint32_t dTmem, const uint8_t *d
                     idesc, (accumulate || j > 0) ? 1u : 0u);
 }
 
-// bias[o] += sum_r dy[r][o] for this tile (fp32 dy)
-__device__ __forceinline__ void accumBias(float *gb, int nOut, const float *dy) {
-    for (int o = threadIdx.x; o < nOut; o += kGTile) {
-        float s = 0.0f;
-        for (int r = 0; r < kGTile; r++) s += dy[r * kTrainStride + o];
-        gb[o] += s;
+// Column sums of the warp's 32 rows, 16 columns, in float32: each step adds the other half of
+// the lanes' values for one half of the columns and hands on the other half, so 16 exchanges do
+// what 16 x 5 would; even lanes add their column to out (a warp's own sums).
+__device__ __forceinline__ void addColumnSums16(const float (&v)[16], float *out) {
+    const int lane = threadIdx.x & 31;
+    float r[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const bool up = lane & 16;
+        r[i] = (up ? v[i + 8] : v[i]) + __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + 8], 16);
     }
+#pragma unroll
+    for (int half = 4; half >= 1; half >>= 1) {
+        const bool up = lane & (2 * half);
+#pragma unroll
+        for (int i = 0; i < half; i++)
+            r[i] = (up ? r[i + half] : r[i]) + __shfl_xor_sync(0xffffffffu, up ? r[i] : r[i + half], 2 * half);
+    }
+    const float sum = r[0] + __shfl_xor_sync(0xffffffffu, r[0], 1);
+    if (!(lane & 1)) out[((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1)] += sum;
 }
 
 // one M = 64 weight-gradient accumulator -> row[offW + o * nIn + i], the CTA's own
@@ -189,20 +199,30 @@ __device__ __forceinline__ void accumBias(float *gb, int nOut, const float *dy) 
 // of each warp hold its rows
 __device__ __forceinline__ void flushWeightGrad(uint32_t dTmem, uint32_t nCols, int offW, int nOut, int nIn,
                                                 float *row) {
+    static_assert(kGParams % 4 == 0 && kOffW2 % 4 == 0 && kOffW3 % 4 == 0 && kOffW4 % 4 == 0, "float4 stores");
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int o = static_cast<int>(16 * warp + lane);
     for (uint32_t c = 0; c < nCols; c += 16) {
         float v[16];
         tc::tmemLoad16(dTmem + ((warp * 32u) << 16) + c, v);
-        if (lane < 16 && o < nOut)
-            for (int i = 0; i < 16; i++)
-                if (static_cast<int>(c) + i < nIn) row[offW + o * nIn + c + i] = v[i];
+        if (lane < 16 && o < nOut) {
+            if (nIn % 16 == 0) {   // whole 16-column pieces of 16-byte aligned rows
+                float4 *dst = reinterpret_cast<float4 *>(row + offW + o * nIn + c);
+#pragma unroll
+                for (int i = 0; i < 4; i++) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i++)
+                    if (static_cast<int>(c) + i < nIn) row[offW + o * nIn + c + i] = v[i];
+            }
+        }
     }
 }
 
-// backward epilogue: g = acc * relu'(h) -> dy (fp32) and dyb (bf16, K = 64); the row's
-// activations come 8 at a time (one core-matrix row, 16 bytes)
-__device__ __forceinline__ void backEpilogue(uint32_t tmem, const uint8_t *h, float *dy, uint8_t *dyb) {
+// backward epilogue: g = acc * relu'(h) -> dyb (bf16, K = 64) and, in float32, its column sums
+// (the layer's bias gradient) into the warp's sums; the row's activations come 8 at a time (one
+// core-matrix row, 16 bytes)
+__device__ __forceinline__ void backEpilogue(uint32_t tmem, const uint8_t *h, float *biasSums, uint8_t *dyb) {
     const uint32_t r = threadIdx.x;
     for (uint32_t c = 0; c < kGHid; c += 16) {
         float v[16];
@@ -219,114 +239,165 @@ __device__ __forceinline__ void backEpilogue(uint32_t tmem, const uint8_t *h, fl
                 a1 = hv.y > 0.0f ? a1 : 0.0f;
             }
         }
-        for (int i = 0; i < 16; i++) dy[r * kTrainStride + c + i] = v[i];
         storeRow8(dyb, r, c, kGHid, v);
         storeRow8(dyb, r, c + 8, kGHid, v + 8);
+        addColumnSums16(v, biasSums + c);
     }
 }
 
+// ring entry of sample s of step's random batch (Philox keyed by (seed, step))
+__device__ __forceinline__ int batchEntry(int s, uint32_t seed, uint32_t step, int avail) {
+    const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>(s), step, 0x47415448u, 0u), make_uint2(seed, 0u));
+    return static_cast<int>(__umulhi(r.x, static_cast<uint32_t>(avail)));
+}
+
+// The gradient of a batch: RING takes sample s from ring entry batchEntry(s) of `samples`, else
+// samples holds the batch.  Bound by latency: one 128-row tile is one chain of eight tensor-core
+// layers and their epilogues per CTA, four warps on its SM.  So what is off the chain goes: the
+// batch is not copied first, its rows and TMEM come while the last step's weights are still
+// being written (dependent launch), bias gradients are summed in registers instead of a serial
+// loop over a float32 tile in shared memory, and the raw outputs never leave the registers.  A
+// step of 16,384 samples, host-timed: 38 us in five launches -> 18.5 us in two (this kernel 24.7
+// -> 17.7 us under ncu).
+template <bool RING>
 __global__ void __launch_bounds__(kGTile, 1) k_guide_train(const uint8_t *__restrict__ packFwd,
                                                            const uint8_t *__restrict__ packBwd,
                                                            const float *__restrict__ biasPad,
-                                                           const float *__restrict__ samples, int n,
-                                                           const float *__restrict__ wsum, float *partials,
-                                                           double *lossAcc, int *err) {
+                                                           const float *__restrict__ samples, int n, int avail,
+                                                           uint32_t seed, uint32_t step, const float *wsum,
+                                                           float *partials, double *lossAcc, int *err) {
     extern __shared__ __align__(128) uint8_t sm[];
     uint8_t *wf = sm + TrainLayout::wf, *wb = sm + TrainLayout::wb;
     float *bias = reinterpret_cast<float *>(sm + TrainLayout::bias);
     uint8_t *x = sm + TrainLayout::x, *h1 = sm + TrainLayout::h1, *h2 = sm + TrainLayout::h2,
             *h3 = sm + TrainLayout::h3, *dyb = sm + TrainLayout::dyb;
-    float *dy = reinterpret_cast<float *>(sm + TrainLayout::dy);
-    float *gb = reinterpret_cast<float *>(sm + TrainLayout::gb);   // bias gradients B1 | B2 | B3 | B4
+    float *gb = reinterpret_cast<float *>(sm + TrainLayout::gb);   // per warp: bias gradients B1 | B2 | B3 | B4
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + TrainLayout::bar);
     uint32_t *tmemSlot = reinterpret_cast<uint32_t *>(sm + TrainLayout::tmem);
     const int t = threadIdx.x;
-    // c is normalised by the batch's weight sum and clamped at 1000x its mean (rare,
-    // bright indirect paths are the signal; only extreme outliers are cut)
-    const float cSum = wsum[0];
-    const float cScale = cSum > 0.0f ? 1.0f / cSum : 0.0f;
-    const float cMax = 1000.0f * cSum / static_cast<float>(n);
     uint64_t *loadBar = reinterpret_cast<uint64_t *>(sm + TrainLayout::loadBar);
-    for (int i = t; i < kBiasPad; i += kGTile) gb[i] = 0.0f;
+    float *myGb = gb + (t >> 5) * kBiasPad;
+    for (int i = t; i < kGTile / 32 * kBiasPad; i += kGTile) gb[i] = 0.0f;
     if (t == 0) {
-        // forward and backward weights and biases: one bulk copy (TMA) each
         tc::mbarInit(bar, 1);
         tc::mbarInit(loadBar, 1);
-        tc::mbarExpectTx(loadBar, kPackFwdBytes + kPackBwdBytes + kBiasPad * 4);
-        tc::bulkLoad(wf, packFwd, kPackFwdBytes, loadBar);
-        tc::bulkLoad(wb, packBwd, kPackBwdBytes, loadBar);
-        tc::bulkLoad(bias, biasPad, kBiasPad * 4, loadBar);
     }
     if (t < 32) {
         tc::tmemAlloc(tmemSlot, kTrainTmemCols);
         tc::tmemRelinquish();
     }
+    // this thread's row of a tile: features, direction and weight (0 past the batch); the ring
+    // does not change while steps run
+    auto loadRow = [&](int tile, float (&xf)[16], float3 &w, float &c) {
+        const int s = tile * kGTile + t;
+#pragma unroll
+        for (int i = 0; i < 16; i++) xf[i] = 0.0f;
+        w = mk(0, 0, 1);
+        c = 0.0f;
+        if (s < n) {
+            const int64_t at = RING ? batchEntry(s, seed, step, avail) : s;
+            const float4 *S = reinterpret_cast<const float4 *>(samples + 16 * at);
+            const float4 q0 = S[0], q1 = S[1], q2 = S[2];
+            xf[0] = q0.x;
+            xf[1] = q0.y;
+            xf[2] = q0.z;
+            xf[3] = q0.w;
+            xf[4] = q1.x;
+            xf[5] = q1.y;
+            xf[6] = q1.z;
+            xf[7] = q1.w;
+            xf[8] = q2.x;
+            w = mk(q2.y, q2.z, q2.w);
+            c = reinterpret_cast<const float *>(S)[12];
+        }
+    };
+    float xf[16];
+    float3 w;
+    float c;
+    loadRow(blockIdx.x, xf, w, c);
+    cudaGridDependencySynchronize();   // the last step's weights and this batch's weight sum
+    cudaTriggerProgrammaticLaunchCompletion();
+    if (t == 0) {
+        // forward and backward weights and biases: one bulk copy (TMA) each
+        tc::mbarExpectTx(loadBar, kPackFwdBytes + kPackBwdBytes + kBiasPad * 4);
+        tc::bulkLoad(wf, packFwd, kPackFwdBytes, loadBar);
+        tc::bulkLoad(wb, packBwd, kPackBwdBytes, loadBar);
+        tc::bulkLoad(bias, biasPad, kBiasPad * 4, loadBar);
+    }
+    // c is normalised by the batch's weight sum and clamped at 1000x its mean (rare,
+    // bright indirect paths are the signal; only extreme outliers are cut)
+    const float cSum = *wsum;
+    const float cScale = cSum > 0.0f ? 1.0f / cSum : 0.0f;
+    const float cMax = 1000.0f * cSum / static_cast<float>(n);
     tc::fenceBeforeSync();
     __syncthreads();
     tc::fenceAfterSync();
     const uint32_t tmem = *tmemSlot;
     uint32_t phase = 0;
     bool ok = bulkLoadWait(loadBar);
-    float lossSum = 0.0f, wSum = 0.0f;
+    float lossSum = 0.0f;
     bool acc = false;   // weight-gradient accumulators hold this CTA's earlier tiles
+    const uint8_t *w1f = wf, *w2f = wf + kW1fBytes, *w3f = w2f + kW2fBytes, *w4f = w3f + kW2fBytes;
     const uint8_t *w2b = wb, *w3b = wb + kW2fBytes, *w4b = wb + 2 * kW2fBytes;
     for (int tile = blockIdx.x; ok && tile * kGTile < n; tile += gridDim.x) {
-        const int s = tile * kGTile + t;
-        float xf[16];
-        float3 w = mk(0, 0, 1);
-        float c = 0.0f;
-        for (int i = 0; i < 16; i++) xf[i] = 0.0f;
-        if (s < n) {
-            const float *S = samples + 16 * static_cast<int64_t>(s);
-            for (int i = 0; i < kGIn; i++) xf[i] = S[i];
-            w = mk(S[9], S[10], S[11]);
-            c = fminf(S[12], cMax) * cScale;
-        }
+        if (acc) loadRow(tile, xf, w, c);
+        c = fminf(c, cMax) * cScale;
         storeRow8(x, t, 0, kGK0, xf);
         storeRow8(x, t, 8, kGK0, xf + 8);
-        ok = mlpForwardTile(tmem, wf, bias, x, h1, h2, h3, dy, kTrainStride, bar, phase);
+        ok = tileMma(tmem, x, w1f, kGK0, kGHid, bar, phase);
+        if (!ok) break;
+        hiddenEpilogue(tmem, bias, h1);
+        ok = tileMma(tmem, h1, w2f, kGHid, kGHid, bar, phase);
+        if (!ok) break;
+        hiddenEpilogue(tmem, bias + kGHid, h2);
+        ok = tileMma(tmem, h2, w3f, kGHid, kGHid, bar, phase);
+        if (!ok) break;
+        hiddenEpilogue(tmem, bias + 2 * kGHid, h3);
+        ok = tileMma(tmem, h3, w4f, kGHid, kGN4, bar, phase);
         if (!ok) break;
         // loss gradient on this thread's row
         {
-            float r[kGOut], g[kGN4];
-            for (int j = 0; j < kGOut; j++) r[j] = dy[t * kTrainStride + j];
-            for (int j = 0; j < kGN4; j++) g[j] = 0.0f;
-            if (s < n && c > 0.0f) {
-                lossSum += mixtureLossGrad(r, w, c, g);
-                wSum += c;
+            float r[kGN4], g[kGN4];
+#pragma unroll
+            for (int k = 0; k < kGN4; k += 16) {
+                float v[16];
+                accRow16(tmem, k, v);
+#pragma unroll
+                for (int i = 0; i < 16; i++) r[k + i] = v[i] + bias[3 * kGHid + k + i];
             }
-            for (int j = 0; j < kGN4; j++) dy[t * kTrainStride + j] = g[j];
+#pragma unroll
+            for (int j = 0; j < kGN4; j++) g[j] = 0.0f;
+            if (c > 0.0f) lossSum += mixtureLossGrad(r, w, c, g);
+#pragma unroll
             for (int j = 0; j < kGN4; j += 8) storeRow8(dyb, t, j, kGN4, g + j);
+#pragma unroll
+            for (int j = 0; j < kGN4; j += 16) {
+                float v[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) v[i] = g[j + i];
+                addColumnSums16(v, myGb + 3 * kGHid + j);
+            }
         }
-        __syncthreads();
-        // each layer: its bias gradient on the CUDA cores, then one commit for the
-        // backward MMA (dX = dY W) and the weight-gradient MMA (dW += dY^T H), which
-        // read the same dY tile
-        accumBias(gb + 3 * kGHid, kGOut, dy);
+        // each layer: one commit for the backward MMA (dX = dY W) and the weight-gradient MMA
+        // (dW += dY^T H), which read the same dY tile
         ok = mmaRun(bar, phase, [&] {
             issueTileMma(tmem, dyb, w4b, kGN4, kGHid);                    // dX3 = dY4 W4
             issueWeightGrad(tmem + kColDW4, dyb, kGN4, h3, kGHid, acc);   // dW4 += dY4^T H3
         });
         if (!ok) break;
-        backEpilogue(tmem, h3, dy, dyb);
-        __syncthreads();
-        accumBias(gb + 2 * kGHid, kGHid, dy);
+        backEpilogue(tmem, h3, myGb + 2 * kGHid, dyb);
         ok = mmaRun(bar, phase, [&] {
             issueTileMma(tmem, dyb, w3b, kGHid, kGHid);                   // dX2 = dY3 W3
             issueWeightGrad(tmem + kColDW3, dyb, kGHid, h2, kGHid, acc);  // dW3 += dY3^T H2
         });
         if (!ok) break;
-        backEpilogue(tmem, h2, dy, dyb);
-        __syncthreads();
-        accumBias(gb + kGHid, kGHid, dy);
+        backEpilogue(tmem, h2, myGb + kGHid, dyb);
         ok = mmaRun(bar, phase, [&] {
             issueTileMma(tmem, dyb, w2b, kGHid, kGHid);                   // dX1 = dY2 W2
             issueWeightGrad(tmem + kColDW2, dyb, kGHid, h1, kGHid, acc);  // dW2 += dY2^T H1
         });
         if (!ok) break;
-        backEpilogue(tmem, h1, dy, dyb);
-        __syncthreads();
-        accumBias(gb, kGHid, dy);
+        backEpilogue(tmem, h1, myGb, dyb);
         ok = mmaRun(bar, phase, [&] {
             issueWeightGrad(tmem + kColDW1, dyb, kGHid, x, kGK0, acc);    // dW1 += dY1^T X
         });
@@ -355,20 +426,14 @@ __global__ void __launch_bounds__(kGTile, 1) k_guide_train(const uint8_t *__rest
     tc::fenceBeforeSync();
     __syncthreads();
     if (t < 32) tc::tmemDealloc(tmem, kTrainTmemCols);
-    for (int o = t; o < kGHid; o += kGTile) {
-        row[kOffB1 + o] = gb[o];
-        row[kOffB2 + o] = gb[kGHid + o];
-        row[kOffB3 + o] = gb[2 * kGHid + o];
-        if (o < kGOut) row[kOffB4 + o] = gb[3 * kGHid + o];
+    for (int o = t; o < kBiasPad; o += kGTile) {
+        const float b = (gb[o] + gb[kBiasPad + o]) + (gb[2 * kBiasPad + o] + gb[3 * kBiasPad + o]);
+        const int layer = o / kGHid, k = o - layer * kGHid;
+        if (layer < 3) row[(layer == 0 ? kOffB1 : layer == 1 ? kOffB2 : kOffB3) + k] = b;
+        else if (k < kGOut) row[kOffB4 + k] = b;
     }
-    for (int off = 16; off > 0; off >>= 1) {
-        lossSum += __shfl_xor_sync(0xffffffffu, lossSum, off);
-        wSum += __shfl_xor_sync(0xffffffffu, wSum, off);
-    }
-    if ((t & 31) == 0) {
-        atomicAdd(&lossAcc[0], static_cast<double>(lossSum));
-        atomicAdd(&lossAcc[1], static_cast<double>(wSum));
-    }
+    for (int off = 16; off > 0; off >>= 1) lossSum += __shfl_xor_sync(0xffffffffu, lossSum, off);
+    if ((t & 31) == 0) atomicAdd(&lossAcc[0], static_cast<double>(lossSum));
 }
 
 // inference only (tests and tools): features [n][9] -> raw outputs [n][40]
@@ -423,55 +488,105 @@ constexpr int kForwardSmem = kPackFwdBytes + kBiasPad * 4 + kGTile * kGK0 * 2 + 
 // ------------------------------------------------------------------ gradient sum, Adam
 // The batch gradient is the sum of the training CTAs' partial rows.  Each block takes
 // kRedX parameters; its kRedY thread rows add every kRedY-th partial row, and the
-// column sums are added in row order, so the sum is the same every time.  ADAM applies
-// an Adam step (Kingma and Ba: bias-corrected moments, c1 = 1 - b1^t, c2 = 1 - b2^t) to
-// the master parameters out with it; otherwise the sum is written to out.
-constexpr int kRedX = 32, kRedY = 8;
-template <bool ADAM>
-__global__ void __launch_bounds__(kRedX *kRedY) k_grad_sum(const float *__restrict__ partials, int nParts, float *out,
-                                                           float *M, float *V, float lr, float b1, float b2, float eps,
-                                                           float c1, float c2) {
-    __shared__ float part[kRedY][kRedX];
-    const int i = blockIdx.x * kRedX + threadIdx.x;
+// column sums are added in row order, so the sum is the same every time.
+constexpr int kRedX = 32, kRedY = 16;
+constexpr int kRedBlocks = (kGParams + kRedX - 1) / kRedX;
+__device__ __forceinline__ float sumPartials(const float *__restrict__ partials, int nParts, int i,
+                                             float (*part)[kRedX]) {
     float s = 0.0f;
-    if (i < kGParams)
+    if (i < kGParams) {
+#pragma unroll 8
         for (int p = threadIdx.y; p < nParts; p += kRedY) s += partials[static_cast<int64_t>(p) * kGParams + i];
+    }
     part[threadIdx.y][threadIdx.x] = s;
     __syncthreads();
-    if (threadIdx.y != 0 || i >= kGParams) return;
     float g = 0.0f;
-    for (int y = 0; y < kRedY; y++) g += part[y][threadIdx.x];
-    if (ADAM) {
-        const float m = b1 * M[i] + (1.0f - b1) * g;
-        const float v = b2 * V[i] + (1.0f - b2) * g * g;
-        M[i] = m;
-        V[i] = v;
-        out[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
-    } else {
-        out[i] = g;
-    }
+    if (threadIdx.y == 0)
+        for (int y = 0; y < kRedY; y++) g += part[y][threadIdx.x];
+    return g;
 }
-constexpr int kRedBlocks = (kGParams + kRedX - 1) / kRedX;
+__global__ void __launch_bounds__(kRedX *kRedY) k_grad_sum(const float *__restrict__ partials, int nParts, float *out) {
+    __shared__ float part[kRedY][kRedX];
+    const int i = blockIdx.x * kRedX + threadIdx.x;
+    const float g = sumPartials(partials, nParts, i, part);
+    if (threadIdx.y == 0 && i < kGParams) out[i] = g;
+}
 
-// gather a random batch of n samples from the first `avail` ring entries (indices from
-// Philox keyed by (seed, step)) and sum their weights
-__global__ void k_gather(const float *ring, int avail, uint32_t seed, uint32_t step, int n, float *batch,
-                         float *wsum) {
+// a block's share of the weight sum of step's random batch
+__device__ __forceinline__ void addBatchWeights(const float *ring, int avail, uint32_t seed, uint32_t step, int n,
+                                                int first, int stride, float *wsum) {
     float part = 0.0f;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
-        const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>(s), step, 0x47415448u, 0u), make_uint2(seed, 0u));
-        const int idx = static_cast<int>(__umulhi(r.x, static_cast<uint32_t>(avail)));
-        const float4 *src = reinterpret_cast<const float4 *>(ring + 16 * static_cast<int64_t>(idx));
-        float4 *dst = reinterpret_cast<float4 *>(batch + 16 * static_cast<int64_t>(s));
-        const float4 q0 = src[0], q1 = src[1], q2 = src[2], q3 = src[3];
-        dst[0] = q0;
-        dst[1] = q1;
-        dst[2] = q2;
-        dst[3] = q3;
-        part += q3.x;   // element 12: the weight c
-    }
+    for (int s = first; s < n; s += stride)
+        part += ring[16 * static_cast<int64_t>(batchEntry(s, seed, step, avail)) + 12];   // element 12: the weight c
     for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-    if ((threadIdx.x & 31) == 0 && part != 0.0f) atomicAdd(&wsum[0], part);
+    if (((threadIdx.y * blockDim.x + threadIdx.x) & 31) == 0 && part != 0.0f) atomicAdd(wsum, part);
+}
+__global__ void k_batch_weights(const float *ring, int avail, uint32_t seed, uint32_t step, int n, float *wsum) {
+    addBatchWeights(ring, avail, seed, step, n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, wsum);
+}
+
+// a parameter's place in the packed operands (k_guide_pack's layout; their padding stays zero)
+__device__ __forceinline__ void packParameter(int i, float v, uint8_t *fwd, uint8_t *bwd, float *biasPad) {
+    auto put = [v](uint8_t *tile, int r, int k, int K) {
+        *reinterpret_cast<__nv_bfloat16 *>(tile + tc::kmajorOffset(r, k, K)) = __float2bfloat16_rn(v);
+    };
+    uint8_t *w2f = fwd + kW1fBytes, *w3f = w2f + kW2fBytes, *w4f = w3f + kW2fBytes;
+    if (i < kOffB1) put(fwd, i / kGIn, i % kGIn, kGK0);
+    else if (i < kOffW2) biasPad[i - kOffB1] = v;
+    else if (i < kOffB2) {
+        const int e = i - kOffW2;
+        put(w2f, e / kGHid, e % kGHid, kGHid);
+        put(bwd, e % kGHid, e / kGHid, kGHid);
+    } else if (i < kOffW3) biasPad[kGHid + i - kOffB2] = v;
+    else if (i < kOffB3) {
+        const int e = i - kOffW3;
+        put(w3f, e / kGHid, e % kGHid, kGHid);
+        put(bwd + kW2fBytes, e % kGHid, e / kGHid, kGHid);
+    } else if (i < kOffW4) biasPad[2 * kGHid + i - kOffB3] = v;
+    else if (i < kOffB4) {
+        const int e = i - kOffW4;
+        put(w4f, e / kGHid, e % kGHid, kGHid);
+        put(bwd + 2 * kW2fBytes, e % kGHid, e / kGHid, kGN4);
+    } else biasPad[3 * kGHid + i - kOffB4] = v;
+}
+
+// The rest of a training step: the gradient's sum, an Adam step (Kingma and Ba: bias-corrected
+// moments, c1 = 1 - b1^t, c2 = 1 - b2^t) on the master parameters, each written to its places in
+// the packed operands, and, in the blocks past kRedBlocks, the weight sum of the next step's batch
+// (wsum[nextSlot]; the slot after that is zeroed for the step after).  One launch instead of four.
+constexpr int kWsumSlots = 3, kWeightBlocks = 16;
+__global__ void __launch_bounds__(kRedX *kRedY) k_step_update(const float *__restrict__ partials, int nParts, float *P,
+                                                              float *M, float *V, float lr, float b1, float b2,
+                                                              float eps, float c1, float c2, uint8_t *fwd, uint8_t *bwd,
+                                                              float *biasPad, const float *ring, int avail,
+                                                              uint32_t seed, uint32_t nextStep, int n, float *wsum,
+                                                              int nextSlot) {
+    __shared__ float part[kRedY][kRedX];
+    if (blockIdx.x >= kRedBlocks) {
+        // the ring does not change while steps run; this slot's last reader was two steps ago
+        const int t = threadIdx.y * kRedX + threadIdx.x, b = blockIdx.x - kRedBlocks;
+        addBatchWeights(ring, avail, seed, nextStep, n, b * kRedX * kRedY + t, kWeightBlocks * kRedX * kRedY,
+                        wsum + nextSlot);
+        cudaGridDependencySynchronize();   // the gradient kernel has read the last slot
+        cudaTriggerProgrammaticLaunchCompletion();
+        if (b == 0 && t == 0) wsum[(nextSlot + 1) % kWsumSlots] = 0.0f;
+        return;
+    }
+    const int i = blockIdx.x * kRedX + threadIdx.x;
+    const bool mine = threadIdx.y == 0 && i < kGParams;
+    // the parameters and moments are the last step's, complete before this step's gradient began
+    const float p0 = mine ? P[i] : 0.0f, m0 = mine ? M[i] : 0.0f, v0 = mine ? V[i] : 0.0f;
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const float g = sumPartials(partials, nParts, i, part);
+    if (!mine) return;
+    const float m = b1 * m0 + (1.0f - b1) * g;
+    const float v = b2 * v0 + (1.0f - b2) * g * g;
+    M[i] = m;
+    V[i] = v;
+    const float p = p0 - lr * (m / c1) / (sqrtf(v / c2) + eps);
+    P[i] = p;
+    packParameter(i, p, fwd, bwd, biasPad);
 }
 
 // weight sum of a caller-supplied batch
@@ -759,7 +874,8 @@ __global__ void __launch_bounds__(kGTile) k_guided(GuidedArgs a) {
 void setGuideKernelAttributes() {
     static std::once_flag once;
     std::call_once(once, [] {
-        cudaFuncSetAttribute(k_guide_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::total);
+        cudaFuncSetAttribute(k_guide_train<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::total);
+        cudaFuncSetAttribute(k_guide_train<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::total);
         cudaFuncSetAttribute(k_guide_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kForwardSmem);
         cudaFuncSetAttribute(k_guided<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGuidedSmem);
         cudaFuncSetAttribute(k_guided<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGuidedSmem);
@@ -799,6 +915,24 @@ int tmemKernelResidentCtas(const void *kernel, int device, int dynSmem = kGuided
     return std::max(1, std::min(std::min(byRegs, bySmem), std::min(std::min(byThreads, blkSM), byTmem)));
 }
 
+// a launch that may begin (up to its cudaGridDependencySynchronize) while the stream's last kernel
+// ends, if dependent
+template <class... Params, class... Args>
+cudaError_t launchDependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool dependent,
+                            Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 template <class T>
 T *galloc(size_t n) {
     T *p = nullptr;
@@ -836,7 +970,6 @@ void freeGuide(GuideState *G) {
     cudaFree(G->ctl);
     cudaFree(G->lossAcc);
     cudaFree(G->wsum);
-    cudaFree(G->batch);
     delete G;
 }
 
@@ -865,10 +998,9 @@ int guideInit(Ctx &C, GuideState **slot, const spgpu_guiding_config *cfg) {
     G->samples = galloc<float>(static_cast<size_t>(G->capacity) * 16);
     G->ctl = galloc<int>(4);
     G->lossAcc = galloc<double>(2);
-    G->wsum = galloc<float>(2);
-    G->batch = galloc<float>(static_cast<size_t>(G->batchCap) * 16);
+    G->wsum = galloc<float>(kWsumSlots);
     if (!G->master || !G->partials || !G->m || !G->v || !G->packFwd || !G->packBwd || !G->biasPad || !G->samples ||
-        !G->ctl || !G->lossAcc || !G->wsum || !G->batch) {
+        !G->ctl || !G->lossAcc || !G->wsum) {
         freeGuide(G);
         setError("spgpu_guiding_init: device allocation failed");
         return SPGPU_ENOMEM;
@@ -934,18 +1066,20 @@ int guideForward(Ctx &C, GuideState &G, const float *feat, int n, float *out, cu
     return 0;
 }
 
-// Launch the gradient of the batch loss (sum_i c_i * -log p(w_i), c normalised by the
-// batch's weight sum in G.wsum[0]): one partial row per training CTA in G.partials,
-// *nParts of them; the c-weighted loss is added to G.lossAcc[0].  No host
-// synchronisation.
-static int launchGrad(Ctx &C, GuideState &G, const float *samples, int n, int *nParts, cudaStream_t s) {
+// Launch the gradient of the batch loss (sum_i c_i * -log p(w_i), c normalised by the batch's
+// weight sum *wsum): one partial row per training CTA in G.partials, *nParts of them; the
+// c-weighted loss is added to G.lossAcc[0].  RING: the batch is drawn from the ring's first
+// `avail` entries, the launch dependent on the stream's last kernel.  No host synchronisation.
+template <bool RING>
+static int launchGrad(Ctx &C, GuideState &G, const float *samples, int n, int avail, uint32_t step, const float *wsum,
+                      int *nParts, cudaStream_t s) {
     const int tiles = (n + kGTile - 1) / kGTile;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, C.device);
     *nParts = std::min(std::min(tiles, sms), G.partialRows);
-    k_guide_train<<<*nParts, kGTile, TrainLayout::total, s>>>(G.packFwd, G.packBwd, G.biasPad, samples, n, G.wsum,
-                                                              G.partials, G.lossAcc, G.ctl + 1);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launchDependent(k_guide_train<RING>, dim3(*nParts), dim3(kGTile), TrainLayout::total, s, RING,
+                                          G.packFwd, G.packBwd, G.biasPad, samples, n, avail, G.cfg.seed, step, wsum,
+                                          G.partials, G.lossAcc, G.ctl + 1);
     return e == cudaSuccess ? 0 : cudaFail("guiding gradient", e);
 }
 
@@ -969,15 +1103,14 @@ int guideGrad(Ctx &C, GuideState &G, const float *samples, int n, float *gradOut
         if (loss) *loss = 0.0;
         return 0;
     }
-    cudaMemsetAsync(G.wsum, 0, 2 * sizeof(float), s);
+    cudaMemsetAsync(G.wsum, 0, kWsumSlots * sizeof(float), s);
     cudaMemsetAsync(G.lossAcc, 0, 2 * sizeof(double), s);
     cudaMemsetAsync(G.ctl + 1, 0, sizeof(int), s);
     k_csum<<<64, 256, 0, s>>>(samples, n, G.wsum);
     int nParts = 0;
-    int rc = launchGrad(C, G, samples, n, &nParts, s);
+    int rc = launchGrad<false>(C, G, samples, n, 0, 0u, G.wsum, &nParts, s);
     if (rc == 0) {
-        k_grad_sum<false><<<kRedBlocks, dim3(kRedX, kRedY), 0, s>>>(G.partials, nParts, gradOut, nullptr, nullptr,
-                                                                    0.0f, 0.0f, 0.0f, 0.0f, 1.0f, 1.0f);
+        k_grad_sum<<<kRedBlocks, dim3(kRedX, kRedY), 0, s>>>(G.partials, nParts, gradOut);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) rc = cudaFail("guiding gradient sum", e);
     }
@@ -1013,21 +1146,24 @@ int guideTrain(Ctx &C, GuideState &G, int steps, double *meanLoss) {
     cudaStream_t s = C.stream;
     cudaMemsetAsync(G.lossAcc, 0, 2 * sizeof(double), s);
     cudaMemsetAsync(G.ctl + 1, 0, sizeof(int), s);
+    cudaMemsetAsync(G.wsum, 0, kWsumSlots * sizeof(float), s);
+    if (steps > 0)
+        k_batch_weights<<<std::min(64, (n + 255) / 256), 256, 0, s>>>(G.samples, avail, G.cfg.seed,
+                                                                       static_cast<uint32_t>(G.step), n, G.wsum);
     for (int st = 0; st < steps; st++) {
-        cudaMemsetAsync(G.wsum, 0, 2 * sizeof(float), s);
-        k_gather<<<std::min(64, (n + 255) / 256), 256, 0, s>>>(G.samples, avail, G.cfg.seed,
-                                                                static_cast<uint32_t>(G.step), n, G.batch, G.wsum);
         int nParts = 0;
-        int rc = launchGrad(C, G, G.batch, n, &nParts, s);
-        if (rc) return rc;
+        const int slot = st % kWsumSlots;
+        if (int rc = launchGrad<true>(C, G, G.samples, n, avail, static_cast<uint32_t>(G.step), G.wsum + slot, &nParts, s))
+            return rc;
         G.step++;
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.0f - std::pow(b1, static_cast<float>(G.step));
         const float c2 = 1.0f - std::pow(b2, static_cast<float>(G.step));
-        k_grad_sum<true><<<kRedBlocks, dim3(kRedX, kRedY), 0, s>>>(G.partials, nParts, G.master, G.m, G.v,
-                                                                   G.cfg.learning_rate, b1, b2, 1.0e-8f, c1, c2);
-        rc = packWeights(G, s);
-        if (rc) return rc;
+        const cudaError_t e = launchDependent(
+            k_step_update, dim3(kRedBlocks + kWeightBlocks), dim3(kRedX, kRedY), 0, s, true, G.partials, nParts, G.master,
+            G.m, G.v, G.cfg.learning_rate, b1, b2, 1.0e-8f, c1, c2, G.packFwd, G.packBwd, G.biasPad, G.samples, avail,
+            G.cfg.seed, static_cast<uint32_t>(G.step), n, G.wsum, (slot + 1) % kWsumSlots);
+        if (e != cudaSuccess) return cudaFail("guiding update", e);
     }
     double lossSum = 0.0;
     const int rc = readLoss(G, &lossSum, s, "spgpu_guiding_train");
