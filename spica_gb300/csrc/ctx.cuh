@@ -138,6 +138,11 @@ struct Ctx {
     std::mutex hostTraceMu;
     unsigned char *hostStage = nullptr;   // rays in, hits out; grown on demand, kept
     size_t hostStageBytes = 0;
+    unsigned char *pinned = nullptr;      // smaller batches' rays, hits and control words, pinned host memory
+    int pinnedRays = 0;                   // rays it holds
+    // spgpu_render_host's film, grown on demand
+    float *hostFilm = nullptr;
+    size_t hostFilmBytes = 0;
     // renderer
     // Render pass lanes: consecutive sample passes alternate between kPassLanes queue
     // sets (each with its own pass graph), lane k > 0 on laneStream[k - 1], so one

@@ -141,3 +141,54 @@ def test_one_class_scene_matches_pass_by_pass(gpulib, cls, width, height, spp):
     x, y = a[..., :3], b[..., :3]
     close = (x - y).abs() <= 1e-5 * y.abs() + 1e-6 * float(y.abs().max())
     assert close.float().mean() > 0.999
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+@pytest.mark.parametrize("rays", [1, 33, 4096, 4097, 65536, 65537, 155647, 155648, 155649])
+def test_ray_batch_routes_agree(gpulib, any_hit, rays):
+    """Host batches up to 65,536 rays are read from and written to pinned host memory, larger ones
+    copied; batches of at most a resident grid's lanes (152 SMs x 8 blocks x 128) take no ray
+    counter.  Host and device entry points give the same records as one 2^18-ray device batch."""
+    import numpy as np
+    import torch
+    acc = GpuBVHAccel(scenes.displaced_sphere(levels=4, seed=3)).construct()
+    org, dirs = _device_rays(1 << 18, 11)
+    shape = (1 << 18,) if any_hit else (1 << 18, 4)
+    if any_hit:
+        dirs[:, 3] = 0.8
+    whole = torch.zeros(shape, dtype=torch.int32, device="cuda")
+    acc.intersect_device(org, dirs, whole, any_hit=any_hit)
+    part = torch.full((rays, *shape[1:]), -7, dtype=torch.int32, device="cuda")
+    for _ in range(2):   # again over the same buffers
+        acc.intersect_device(org[:rays], dirs[:rays], part, any_hit=any_hit)
+    torch.cuda.synchronize()
+    assert torch.equal(part, whole[:rays])
+    o, d = org[:rays].cpu().numpy(), dirs[:rays].cpu().numpy()
+    want = whole[:rays].cpu().numpy()
+    for _ in range(2):
+        if any_hit:
+            np.testing.assert_array_equal(acc.intersect_any(o[:, :3], d[:, :3], d[:, 3]), want.astype(bool))
+        else:
+            prim, t, u, v = acc.intersect(o[:, :3], d[:, :3], d[:, 3])
+            np.testing.assert_array_equal(prim, want[:, 1])
+            for got, k in ((t, 0), (u, 2), (v, 3)):
+                np.testing.assert_array_equal(got.view(np.int32), want[:, k])
+
+
+def test_host_films_of_changing_size(gpulib):
+    """Host renders through the context's kept film buffer, growing and shrinking, add to the
+    caller's film as the device entry point adds to a device film (the order of the additions of
+    four samples: 1e-6 relative)."""
+    import numpy as np
+    import torch
+    from spica_gb300 import GpuPathIntegrator
+    sc = scenes.box_room(width=32, height=32)
+    acc = GpuBVHAccel(sc).construct()
+    integ = GpuPathIntegrator(seed=4)
+    for w, h in ((16, 8), (64, 48), (5, 3), (64, 49)):
+        p = {"width": w, "height": h, "maxDepth": 4, "sampleCount": 4}
+        host = integ.render(sc.camera, acc, p, film=np.full((h, w, 4), 0.5, np.float32))
+        dev = torch.full((h, w, 4), 0.5, device="cuda")
+        integ.render_device(sc.camera, acc, p, dev)
+        np.testing.assert_allclose(host, dev.cpu().numpy(), rtol=1e-6, atol=1e-6)
+        assert np.all(host[..., 3] == 4.5)
