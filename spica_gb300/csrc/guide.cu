@@ -29,7 +29,7 @@ struct GuideState {
     int capacity = 0;
     int *ctl = nullptr;         // [0] samples written (monotonic), [1] error, [2] work counter
     double *lossAcc = nullptr;  // [0] loss sum, [1] weight sum
-    float *wsum = nullptr;      // batch weight sums: of this step, the next and the last (kWsumSlots)
+    double *wsum = nullptr;     // batch weight sums: of this step, the next and the last (kWsumSlots)
     int batchCap = 0;
     float *partials = nullptr;  // per training CTA: its partial gradient (kGParams floats)
     int partialRows = 0;
@@ -251,20 +251,19 @@ __device__ __forceinline__ int batchEntry(int s, uint32_t seed, uint32_t step, i
     return static_cast<int>(__umulhi(r.x, static_cast<uint32_t>(avail)));
 }
 
-// The gradient of a batch: RING takes sample s from ring entry batchEntry(s) of `samples`, else
-// samples holds the batch.  Bound by latency: one 128-row tile is one chain of eight tensor-core
+// The gradient of a batch: with avail > 0, sample s is ring entry batchEntry(s) of `samples`, else
+// samples holds the batch (one kernel for both, so that both round alike).  Bound by latency: one 128-row tile is one chain of eight tensor-core
 // layers and their epilogues per CTA, four warps on its SM.  So what is off the chain goes: the
 // batch is not copied first, its rows and TMEM come while the last step's weights are still
 // being written (dependent launch), bias gradients are summed in registers instead of a serial
 // loop over a float32 tile in shared memory, and the raw outputs never leave the registers.  A
 // step of 16,384 samples, host-timed: 38 us in five launches -> 18.5 us in two (this kernel 24.7
 // -> 17.7 us under ncu).
-template <bool RING>
 __global__ void __launch_bounds__(kGTile, 1) k_guide_train(const uint8_t *__restrict__ packFwd,
                                                            const uint8_t *__restrict__ packBwd,
                                                            const float *__restrict__ biasPad,
                                                            const float *__restrict__ samples, int n, int avail,
-                                                           uint32_t seed, uint32_t step, const float *wsum,
+                                                           uint32_t seed, uint32_t step, const double *wsum,
                                                            float *partials, double *lossAcc, int *err) {
     extern __shared__ __align__(128) uint8_t sm[];
     uint8_t *wf = sm + TrainLayout::wf, *wb = sm + TrainLayout::wb;
@@ -295,7 +294,7 @@ __global__ void __launch_bounds__(kGTile, 1) k_guide_train(const uint8_t *__rest
         w = mk(0, 0, 1);
         c = 0.0f;
         if (s < n) {
-            const int64_t at = RING ? batchEntry(s, seed, step, avail) : s;
+            const int64_t at = avail > 0 ? batchEntry(s, seed, step, avail) : s;
             const float4 *S = reinterpret_cast<const float4 *>(samples + 16 * at);
             const float4 q0 = S[0], q1 = S[1], q2 = S[2];
             xf[0] = q0.x;
@@ -326,7 +325,7 @@ __global__ void __launch_bounds__(kGTile, 1) k_guide_train(const uint8_t *__rest
     }
     // c is normalised by the batch's weight sum and clamped at 1000x its mean (rare,
     // bright indirect paths are the signal; only extreme outliers are cut)
-    const float cSum = *wsum;
+    const float cSum = static_cast<float>(*wsum);
     const float cScale = cSum > 0.0f ? 1.0f / cSum : 0.0f;
     const float cMax = 1000.0f * cSum / static_cast<float>(n);
     tc::fenceBeforeSync();
@@ -512,16 +511,17 @@ __global__ void __launch_bounds__(kRedX *kRedY) k_grad_sum(const float *__restri
     if (threadIdx.y == 0 && i < kGParams) out[i] = g;
 }
 
-// a block's share of the weight sum of step's random batch
+// a block's share of the weight sum of step's random batch.  In double, so that its float32
+// value does not depend on the order of the additions (nor a batch's gradient on who asks)
 __device__ __forceinline__ void addBatchWeights(const float *ring, int avail, uint32_t seed, uint32_t step, int n,
-                                                int first, int stride, float *wsum) {
-    float part = 0.0f;
+                                                int first, int stride, double *wsum) {
+    double part = 0.0;
     for (int s = first; s < n; s += stride)
         part += ring[16 * static_cast<int64_t>(batchEntry(s, seed, step, avail)) + 12];   // element 12: the weight c
     for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-    if (((threadIdx.y * blockDim.x + threadIdx.x) & 31) == 0 && part != 0.0f) atomicAdd(wsum, part);
+    if (((threadIdx.y * blockDim.x + threadIdx.x) & 31) == 0 && part != 0.0) atomicAdd(wsum, part);
 }
-__global__ void k_batch_weights(const float *ring, int avail, uint32_t seed, uint32_t step, int n, float *wsum) {
+__global__ void k_batch_weights(const float *ring, int avail, uint32_t seed, uint32_t step, int n, double *wsum) {
     addBatchWeights(ring, avail, seed, step, n, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, wsum);
 }
 
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kRedX *kRedY) k_step_update(const float *__res
                                                               float *M, float *V, float lr, float b1, float b2,
                                                               float eps, float c1, float c2, uint8_t *fwd, uint8_t *bwd,
                                                               float *biasPad, const float *ring, int avail,
-                                                              uint32_t seed, uint32_t nextStep, int n, float *wsum,
+                                                              uint32_t seed, uint32_t nextStep, int n, double *wsum,
                                                               int nextSlot) {
     __shared__ float part[kRedY][kRedX];
     if (blockIdx.x >= kRedBlocks) {
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(kRedX *kRedY) k_step_update(const float *__res
                         wsum + nextSlot);
         cudaGridDependencySynchronize();   // the gradient kernel has read the last slot
         cudaTriggerProgrammaticLaunchCompletion();
-        if (b == 0 && t == 0) wsum[(nextSlot + 1) % kWsumSlots] = 0.0f;
+        if (b == 0 && t == 0) wsum[(nextSlot + 1) % kWsumSlots] = 0.0;
         return;
     }
     const int i = blockIdx.x * kRedX + threadIdx.x;
@@ -590,12 +590,12 @@ __global__ void __launch_bounds__(kRedX *kRedY) k_step_update(const float *__res
 }
 
 // weight sum of a caller-supplied batch
-__global__ void k_csum(const float *samples, int n, float *wsum) {
-    float part = 0.0f;
+__global__ void k_csum(const float *samples, int n, double *wsum) {
+    double part = 0.0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
         part += samples[16 * static_cast<int64_t>(s) + 12];
     for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
-    if ((threadIdx.x & 31) == 0 && part != 0.0f) atomicAdd(&wsum[0], part);
+    if ((threadIdx.x & 31) == 0 && part != 0.0) atomicAdd(&wsum[0], part);
 }
 
 // ------------------------------------------------------------------ guided tracer
@@ -874,8 +874,7 @@ __global__ void __launch_bounds__(kGTile) k_guided(GuidedArgs a) {
 void setGuideKernelAttributes() {
     static std::once_flag once;
     std::call_once(once, [] {
-        cudaFuncSetAttribute(k_guide_train<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::total);
-        cudaFuncSetAttribute(k_guide_train<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::total);
+        cudaFuncSetAttribute(k_guide_train, cudaFuncAttributeMaxDynamicSharedMemorySize, TrainLayout::total);
         cudaFuncSetAttribute(k_guide_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kForwardSmem);
         cudaFuncSetAttribute(k_guided<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGuidedSmem);
         cudaFuncSetAttribute(k_guided<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGuidedSmem);
@@ -998,7 +997,7 @@ int guideInit(Ctx &C, GuideState **slot, const spgpu_guiding_config *cfg) {
     G->samples = galloc<float>(static_cast<size_t>(G->capacity) * 16);
     G->ctl = galloc<int>(4);
     G->lossAcc = galloc<double>(2);
-    G->wsum = galloc<float>(kWsumSlots);
+    G->wsum = galloc<double>(kWsumSlots);
     if (!G->master || !G->partials || !G->m || !G->v || !G->packFwd || !G->packBwd || !G->biasPad || !G->samples ||
         !G->ctl || !G->lossAcc || !G->wsum) {
         freeGuide(G);
@@ -1068,16 +1067,15 @@ int guideForward(Ctx &C, GuideState &G, const float *feat, int n, float *out, cu
 
 // Launch the gradient of the batch loss (sum_i c_i * -log p(w_i), c normalised by the batch's
 // weight sum *wsum): one partial row per training CTA in G.partials, *nParts of them; the
-// c-weighted loss is added to G.lossAcc[0].  RING: the batch is drawn from the ring's first
+// c-weighted loss is added to G.lossAcc[0].  avail > 0: the batch is drawn from the ring's first
 // `avail` entries, the launch dependent on the stream's last kernel.  No host synchronisation.
-template <bool RING>
-static int launchGrad(Ctx &C, GuideState &G, const float *samples, int n, int avail, uint32_t step, const float *wsum,
+static int launchGrad(Ctx &C, GuideState &G, const float *samples, int n, int avail, uint32_t step, const double *wsum,
                       int *nParts, cudaStream_t s) {
     const int tiles = (n + kGTile - 1) / kGTile;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, C.device);
     *nParts = std::min(std::min(tiles, sms), G.partialRows);
-    const cudaError_t e = launchDependent(k_guide_train<RING>, dim3(*nParts), dim3(kGTile), TrainLayout::total, s, RING,
+    const cudaError_t e = launchDependent(k_guide_train, dim3(*nParts), dim3(kGTile), TrainLayout::total, s, avail > 0,
                                           G.packFwd, G.packBwd, G.biasPad, samples, n, avail, G.cfg.seed, step, wsum,
                                           G.partials, G.lossAcc, G.ctl + 1);
     return e == cudaSuccess ? 0 : cudaFail("guiding gradient", e);
@@ -1103,12 +1101,12 @@ int guideGrad(Ctx &C, GuideState &G, const float *samples, int n, float *gradOut
         if (loss) *loss = 0.0;
         return 0;
     }
-    cudaMemsetAsync(G.wsum, 0, kWsumSlots * sizeof(float), s);
+    cudaMemsetAsync(G.wsum, 0, kWsumSlots * sizeof(double), s);
     cudaMemsetAsync(G.lossAcc, 0, 2 * sizeof(double), s);
     cudaMemsetAsync(G.ctl + 1, 0, sizeof(int), s);
     k_csum<<<64, 256, 0, s>>>(samples, n, G.wsum);
     int nParts = 0;
-    int rc = launchGrad<false>(C, G, samples, n, 0, 0u, G.wsum, &nParts, s);
+    int rc = launchGrad(C, G, samples, n, 0, 0u, G.wsum, &nParts, s);
     if (rc == 0) {
         k_grad_sum<<<kRedBlocks, dim3(kRedX, kRedY), 0, s>>>(G.partials, nParts, gradOut);
         const cudaError_t e = cudaGetLastError();
@@ -1146,14 +1144,14 @@ int guideTrain(Ctx &C, GuideState &G, int steps, double *meanLoss) {
     cudaStream_t s = C.stream;
     cudaMemsetAsync(G.lossAcc, 0, 2 * sizeof(double), s);
     cudaMemsetAsync(G.ctl + 1, 0, sizeof(int), s);
-    cudaMemsetAsync(G.wsum, 0, kWsumSlots * sizeof(float), s);
+    cudaMemsetAsync(G.wsum, 0, kWsumSlots * sizeof(double), s);
     if (steps > 0)
         k_batch_weights<<<std::min(64, (n + 255) / 256), 256, 0, s>>>(G.samples, avail, G.cfg.seed,
                                                                        static_cast<uint32_t>(G.step), n, G.wsum);
     for (int st = 0; st < steps; st++) {
         int nParts = 0;
         const int slot = st % kWsumSlots;
-        if (int rc = launchGrad<true>(C, G, G.samples, n, avail, static_cast<uint32_t>(G.step), G.wsum + slot, &nParts, s))
+        if (int rc = launchGrad(C, G, G.samples, n, avail, static_cast<uint32_t>(G.step), G.wsum + slot, &nParts, s))
             return rc;
         G.step++;
         const float b1 = 0.9f, b2 = 0.999f;
