@@ -128,6 +128,7 @@ struct StreamArgs {
     // of the iteration whose shadow rays k_strace traces (null: none)
     int onePass;
     int *shadowCtr;
+    int besideLast, besideNext;   // k_sshade: runs beside the last / next kernel (launchShading)
     // guided renders: the network's packed weights and biases (null: plain BSDF
     // sampling), the proposal's BSDF share, the depths that sample it (0: all but the
     // last), and the scene box that normalises the network's position input
@@ -366,6 +367,20 @@ __device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const Shad
     }
 }
 
+// First statement of the shading kernels (launchShading): a class that runs beside the last
+// kernel does not wait for it, and one that lets the next run beside it does so only once what
+// both depend on is complete.
+__device__ __forceinline__ void beginShading(const StreamArgs &p) {
+    if (p.besideLast) {
+        cudaTriggerProgrammaticLaunchCompletion();
+    } else if (p.besideNext) {
+        cudaGridDependencySynchronize();
+        cudaTriggerProgrammaticLaunchCompletion();
+    } else {
+        awaitLastKernel();
+    }
+}
+
 // the rows that class cls shades in this iteration: its queue, or the pool's rays where the
 // scene has that class alone
 struct ShadeRows {
@@ -400,7 +415,7 @@ __device__ __forceinline__ HitRecord hitOfRow(float4 h4) {
 // at 333 x 217 (24 samples) 1.94 -> 1.81 ms.
 template <int CLS, bool BATCH>
 __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(StreamArgs p) {
-    awaitLastKernel();
+    beginShading(p);
     const ShadeRows rows = shadeRows(p, CLS);
     const int n = rows.n;
     const int stride = gridDim.x * blockDim.x;
@@ -448,6 +463,7 @@ __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(St
         }
         emitShadeResultS<BATCH>(p, R, live, filmIdx, pix, meta, sample);
     }
+    if (p.besideLast) cudaGridDependencySynchronize();
 }
 
 // Lambert hits of a guided render.  Each CTA takes 128-row tiles of the Lambert queue:
@@ -458,7 +474,7 @@ __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(St
 // mixes depths, so one launch covers what the pass-by-pass wavefront does in one guided
 // launch per bounce.
 __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(StreamArgs p) {
-    awaitLastKernel();
+    beginShading(p);
     const ShadeRows rows = shadeRows(p, kMatLambert);
     const int n = rows.n;
     if (static_cast<int>(blockIdx.x) * kGTile >= n) return;   // no tile for this CTA
@@ -707,23 +723,28 @@ StreamArgs poolsSwapped(StreamArgs a) {
     return a;
 }
 
-// the shading kernels of the classes in mask; returns how many
+// The shading kernels of the classes in mask; returns how many.  In one-pass renders they run
+// beside each other: they depend on the extend before them, not on one another.  The first waits
+// for it and then lets the second begin, which lets the third begin at once; each of these ends
+// only after the one before it, so whatever follows the last follows all.  Small queues' rows
+// take long (a rough dielectric's five evaluations and its iterated slope inversion), so the
+// glossy class goes first: the conductor room at 281 x 159 (15 samples) 0.77 -> 0.70 ms, the
+// material room at 100 x 80 (4) 0.52 -> 0.49, the mid-scale scene at 1080p (8) 13.4 -> 13.1.
 template <bool BATCH>
 int launchShading(const StreamArgs &a, const GridsS &g, cudaStream_t s, int mask) {
+    const int total = (mask & 1) + (mask >> 1 & 1) + (mask >> 2 & 1);
     int n = 0;
-    if (mask & 1) {
-        if (a.packFwd) launchStreamKernel(k_sshade_guided, g.guided, kGTile, kGsSmem, s, a);
-        else launchStreamKernel(k_sshade<0, BATCH>, g.shade, kShadeBlockS, 0, s, a);
+    StreamArgs p = a;
+    auto launch = [&](auto kernel, int grid, int block, size_t smem) {
+        p.besideLast = a.onePass && n > 0;
+        p.besideNext = a.onePass && n + 1 < total;
+        launchStreamKernel(kernel, grid, block, smem, s, p);
         n++;
-    }
-    if (mask & 2) {
-        launchStreamKernel(k_sshade<1, BATCH>, g.shade, kShadeBlockS, 0, s, a);
-        n++;
-    }
-    if (mask & 4) {
-        launchStreamKernel(k_sshade<2, BATCH>, g.shade, kShadeBlockS, 0, s, a);
-        n++;
-    }
+    };
+    if ((mask & 1) && a.packFwd) launch(k_sshade_guided, g.guided, kGTile, kGsSmem);
+    if (mask & 2) launch(k_sshade<1, BATCH>, g.shade, kShadeBlockS, 0);
+    if (mask & 4) launch(k_sshade<2, BATCH>, g.shade, kShadeBlockS, 0);
+    if ((mask & 1) && !a.packFwd) launch(k_sshade<0, BATCH>, g.shade, kShadeBlockS, 0);
     return n;
 }
 
@@ -1167,10 +1188,15 @@ void freeStreamQueues(StreamQueues *q) {
 
 namespace {
 
-// Paths up to which a one-pass render takes a single lane.  Two lanes' kernels overlap, but
-// each has its own launches: one lane / two, 66k paths 0.43 / 0.46 ms, 1.7M paths in the
-// material room 1.37 / 1.32 ms, 1.8M guided 3.31 / 3.32 ms.
-constexpr long long kOneLanePaths = 1 << 18;
+// Paths up to which a one-pass render takes a single lane.  Two lanes' kernels overlap, but each
+// has its own launches, and they take turns on the chip; several classes, which run beside each
+// other, and guided shading fill it alone for longer.  One lane / two: box room, 393k paths 0.419
+// / 0.427 ms, 720k 0.500 / 0.490, 1M 0.620 / 0.601; mid-scale scene, 518k 1.95 / 2.74; conductor
+// room, 670k 0.70 / 0.76; material room, 1.7M 1.39 / 1.31; guided room, 460k 1.37 / 1.47, 922k
+// 1.95 / 2.01, 1.8M 3.31 / 3.32.
+long long oneLanePaths(const StreamArgs &a) {
+    return a.singleClass >= 0 && !a.packFwd ? 1 << 19 : 1 << 20;
+}
 
 // A render whose paths all fit the pools' slots at once.  Every path starts in the first
 // iteration and iteration b handles depth b, so the iterations are known beforehand: no refill,
@@ -1185,8 +1211,10 @@ int renderOnePass(Ctx &C, const float *camera, int W, int H, int spp, int sample
                   int integrator, float4 *film, unsigned long long *statsOut, float *msOut, cudaStream_t stream,
                   const GuideView *gv) {
     const long long total = static_cast<long long>(W) * H * spp;
-    const int lanes = total <= kOneLanePaths ? 1 : std::max(1, std::min(spp, Ctx::kPoolLanes));
-    StreamArgs a[Ctx::kPoolLanes];
+    StreamArgs a[Ctx::kPoolLanes] = {};
+    setPools(a[0], C.classMask);
+    a[0].packFwd = gv ? gv->packFwd : nullptr;
+    const int lanes = total <= oneLanePaths(a[0]) ? 1 : std::max(1, std::min(spp, Ctx::kPoolLanes));
     StreamInit init[Ctx::kPoolLanes];
     cudaStream_t ls[Ctx::kPoolLanes];
     int first = sampleOffset;

@@ -48,9 +48,11 @@ ROOMS = {"box": scenes.box_room, "material": scenes.material_room, "conductor": 
     ("box", 33, 17, 1, 64, "path"),          # one sample; deeper than the iterations between two looks
     ("material", 64, 48, 5, 17, "path"),     # all classes; odd samples; one iteration past a look
     ("conductor", 40, 30, 3, 16, "path"),
-    ("box", 512, 512, 1, 3, "path"),         # 2^18 paths: the last in one lane
-    ("box", 512, 513, 1, 3, "path"),         # one sample cannot be shared
-    ("material", 512, 257, 3, 3, "path"),    # two lanes, uneven shares
+    ("box", 512, 512, 2, 3, "path"),         # 2^19 paths: the last of one class in one lane
+    ("box", 512, 513, 2, 3, "path"),
+    ("box", 1024, 1025, 1, 3, "path"),       # one sample cannot be shared
+    ("material", 512, 512, 4, 3, "path"),    # 2^20 paths: the last in one lane
+    ("material", 512, 513, 5, 3, "path"),    # two lanes, uneven shares
     ("material", 65, 31, 4, 5, "direct"),
 ])
 def test_one_pass_render_matches_pass_by_pass(gpulib, room, width, height, spp, depth, integrator):
