@@ -670,6 +670,7 @@ void spgpu_destroy(spgpu_ctx *h) {
     cudaFree(C.traceStats);
     cudaFree(C.hostStage);
     cudaFree(C.hostFilm);
+    cudaFree(C.filmScratch);
     if (C.pinned) cudaFreeHost(C.pinned);
     if (C.stream) cudaStreamDestroy(C.stream);
     delete h;
@@ -1277,6 +1278,7 @@ int spgpu_render_host(spgpu_ctx *h, const spgpu_render_desc *d, float *film, spg
         if (kept) {
             if (C.hostFilmBytes < bytes) {
                 cudaFree(C.hostFilm);
+    cudaFree(C.filmScratch);
                 C.hostFilm = nullptr;
                 C.hostFilmBytes = 0;
                 e = cudaMalloc(&C.hostFilm, bytes);

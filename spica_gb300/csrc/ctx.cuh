@@ -143,6 +143,10 @@ struct Ctx {
     // spgpu_render_host's film, grown on demand
     float *hostFilm = nullptr;
     size_t hostFilmBytes = 0;
+    // spgpu_film_resolve's scratch, grown on demand
+    std::mutex filmScratchMu;
+    unsigned char *filmScratch = nullptr;
+    size_t filmScratchBytes = 0;
     // renderer
     // Render pass lanes: consecutive sample passes alternate between kPassLanes queue
     // sets (each with its own pass graph), lane k > 0 on laneStream[k - 1], so one

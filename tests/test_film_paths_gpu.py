@@ -100,3 +100,23 @@ def test_durand_non_finite_pixel(gpulib):
     with np.errstate(all="ignore"):
         want = tmo_oracle.durand(film, 5.0)
     np.testing.assert_array_equal(_resolve(film, gpu.FILM_DURAND, 5.0), want)
+
+
+@pytest.mark.parametrize("odd", [None, (0.0, 0.0, 0.0, 0.0), (-1.0, 0.2, 0.1, 1.0), (1.0, 2.0, 3.0, 0.0),
+                                 (np.inf, 1.0, 1.0, 4.0), (1.0, np.nan, 1.0, 4.0)])
+@pytest.mark.parametrize("param", [0.18, 0.5, 0.85, 1.0, 1.7])
+def test_reinhard_and_drago_with_odd_pixels(gpulib, param, odd):
+    """The operators' reduced FP64 arithmetic on films over six decades, with black pixels and one
+    unusual one (a negative, infinite or NaN channel, no weight), against the restatement (2e-6
+    relative, as in test_film_gpu.py; the same values not finite)."""
+    from oracle import tmo_oracle
+    from spica_gb300 import gpu
+    rng = np.random.default_rng(9)
+    film = np.concatenate([rng.lognormal(0, 2.5, (37, 53, 3)), np.full((37, 53, 1), 4.0)], -1).astype(np.float32)
+    film[rng.random((37, 53)) < 0.05, :3] = 0.0
+    if odd is not None:
+        film[20, 31] = odd
+    for fmt, op in ((gpu.FILM_REINHARD, tmo_oracle.reinhard), (gpu.FILM_DRAGO, tmo_oracle.drago)):
+        with np.errstate(all="ignore"):
+            want = op(film, param).astype(np.float32)
+        np.testing.assert_allclose(_resolve(film, fmt, param), want, rtol=2e-6, atol=1e-30)
