@@ -30,7 +30,7 @@
 // A build was bound by what surrounds its kernels: some 75 clustering rounds of eight launches
 // and a host round trip each, 30 allocations, and one thread per wide node in the collapse.  With
 // rounds that run ahead of the host, the last rounds in one block, one scratch allocation and
-// eight threads per wide node, 2.03M triangles take 11.4 -> 3.5 ms, 256 triangles 1.96 -> 0.28.
+// eight threads per wide node, 2.03M triangles take 11.4 -> 3.2 ms, 256 triangles 1.96 -> 0.28.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
@@ -187,6 +187,11 @@ __global__ void k_leaf_bounds(const float *__restrict__ verts, const uint32_t *_
 // kRoundsAhead rounds, sized by the last count it knows, between two looks.  From kTailClusters
 // clusters on, one block does the rest (k_ploc_tail): with 4096 / 2048 / 1024 / 512 of them the
 // 2M-triangle build takes 3.50 / 3.48 / 3.47 / 3.60 ms, 16k triangles 1.12 / 1.08 / 1.10 / 1.16.
+// A round is three kernels of a few microseconds, so they are dependent launches: each is set up
+// while the one before it runs, and waits for it before its first access.  A round's SAH
+// programme runs beside the next round's counting (and the last round's in k_ploc_tail).  Both
+// together, and the collapse's levels as dependent launches: 2M triangles 3.53 -> 3.16 ms, 16k
+// 1.09 -> 0.98 ms.
 struct RoundState {
     int m, top;
 };
@@ -203,6 +208,8 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const int *__restrict__ 
                                                         const float4 *__restrict__ bmin,
                                                         const float4 *__restrict__ bmax, int *nn) {
     __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius], shi[kPlocBlock + 2 * kPlocRadius];
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     const int m = round->m;
     if (m <= kTailClusters || static_cast<int>(blockIdx.x) * kPlocBlock >= m) return;
     const int base = blockIdx.x * kPlocBlock - kPlocRadius;
@@ -264,19 +271,6 @@ __device__ __forceinline__ uint32_t countBefore(bool lead, bool keep, uint32_t *
 }
 static_assert(kMergeBlock == 1024, "32 warps, a lane for each in countBefore; counts of 16 bits");
 
-// leads and survivors of each block of kMergeBlock clusters
-__global__ void __launch_bounds__(kMergeBlock) k_ploc_count(const int *__restrict__ nn,
-                                                            const RoundState *__restrict__ round, uint32_t *sums) {
-    __shared__ uint32_t warpSum[32];
-    const int m = round->m;
-    if (m <= kTailClusters || static_cast<int>(blockIdx.x) * kMergeBlock >= m) return;
-    bool lead, keep;
-    mergeFlags(nn, blockIdx.x * kMergeBlock + threadIdx.x, m, &lead, &keep);
-    uint32_t total;
-    countBefore(lead, keep, warpSum, &total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
-}
-
 // merged nodes take ids top - (leads before) (descending, so the last merge, the root, is node
 // 0); survivors are compacted in order.  Each block adds up the counts of the blocks before it.
 __global__ void __launch_bounds__(kMergeBlock) k_ploc_merge(const int *__restrict__ clusters, RoundState *round,
@@ -285,6 +279,8 @@ __global__ void __launch_bounds__(kMergeBlock) k_ploc_merge(const int *__restric
                                                             float4 *bmin, float4 *bmax, int *count, int *next) {
     __shared__ uint32_t warpSum[32];
     __shared__ int base[2];
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     const int m = round->m, top = round->top;
     if (static_cast<int>(blockIdx.x) * kMergeBlock >= m) return;
     if (m <= kTailClusters) {   // nothing left for the rounds: clusters and state go on to the tail
@@ -402,24 +398,51 @@ __device__ __forceinline__ void dpNode(const DpArgs &D, int n, int id, int2 c, i
     D.leaf[id] = asLeaf ? 1 : 0;
 }
 
-// one clustering round's nodes (round[1].top < id <= round[0].top; their children are from
-// earlier rounds)
-__global__ void k_dp_round(const int2 *__restrict__ child, const int *__restrict__ count,
-                           const float4 *__restrict__ bmin, const float4 *__restrict__ bmax,
-                           const RoundState *__restrict__ round, int n, DpArgs D) {
-    const int id = round[1].top + 1 + static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    if (id > round[0].top) return;
-    dpNode(D, n, id, child[id], count[id], bmin[id], bmax[id], bmin, bmax);
+// the SAH programme of the nodes that the round before this one merged (round[0].top < id <=
+// round[-1].top; their children are from earlier rounds), thread by thread of stride threads
+__device__ __forceinline__ void dpLastRound(const DpArgs &D, int n, const RoundState *round, int thread, int stride,
+                                            const int2 *child, const int *count, const float4 *bmin,
+                                            const float4 *bmax) {
+    const int last = round[-1].top;
+    for (int id = round[0].top + 1 + thread; id <= last; id += stride)
+        dpNode(D, n, id, child[id], count[id], bmin[id], bmax[id], bmin, bmax);
+}
+
+// Leads and survivors of each block of kMergeBlock clusters, and beside them, in the launch's
+// first dpBlocks blocks, the last round's SAH programme: both wait on memory most of the time,
+// and apart they were 4 and 6 us a round of a 2M-triangle build, with a launch each.
+__global__ void __launch_bounds__(kMergeBlock) k_ploc_count(const int *__restrict__ nn,
+                                                            const RoundState *__restrict__ round, uint32_t *sums,
+                                                            int dpBlocks, const int2 *__restrict__ child,
+                                                            const int *__restrict__ count,
+                                                            const float4 *__restrict__ bmin,
+                                                            const float4 *__restrict__ bmax, int n, DpArgs D) {
+    __shared__ uint32_t warpSum[32];
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int block = static_cast<int>(blockIdx.x) - dpBlocks;
+    if (block < 0) {
+        dpLastRound(D, n, round, blockIdx.x * kMergeBlock + threadIdx.x, dpBlocks * kMergeBlock, child, count, bmin, bmax);
+        return;
+    }
+    const int m = round->m;
+    if (m <= kTailClusters || block * kMergeBlock >= m) return;
+    bool lead, keep;
+    mergeFlags(nn, block * kMergeBlock + threadIdx.x, m, &lead, &keep);
+    uint32_t total;
+    countBefore(lead, keep, warpSum, &total);
+    if (threadIdx.x == 0) sums[block] = total;
 }
 
 // The clustering's last rounds, with their SAH programme, in one block: at most kTailClusters
 // clusters, whose boxes stay in shared memory.  A round of a few thousand clusters is too little
 // for the chip and its launches cost more than its work; there are some forty of them.
-// state: in, the clusters and next free id; out, what is left (one cluster, top -1).
+// state: in, the clusters and next free id; out, what is left (one cluster, top -1).  After
+// rounds of their own kernels (rounds true) the last one's SAH programme comes first.
 constexpr int kTailSmem = kTailClusters * (2 * static_cast<int>(sizeof(float4)) + static_cast<int>(sizeof(int)));
 __global__ void __launch_bounds__(kMergeBlock) k_ploc_tail(const int *__restrict__ clusters, RoundState *state,
                                                            int2 *child, float4 *bmin, float4 *bmax, int *count, int n,
-                                                           DpArgs D) {
+                                                           bool rounds, DpArgs D) {
     extern __shared__ float4 box[];   // per cluster: lo (w: node id), hi (w: triangles)
     __shared__ uint32_t warpSum[32];
     float4 *slo = box, *shi = box + kTailClusters;
@@ -427,6 +450,7 @@ __global__ void __launch_bounds__(kMergeBlock) k_ploc_tail(const int *__restrict
     int m = state->m, top = state->top;
     if (m > kTailClusters) return;
     const int t = threadIdx.x;
+    if (rounds) dpLastRound(D, n, state, t, kMergeBlock, child, count, bmin, bmax);   // complete at the barrier below
     for (int i = t; i < m; i += kMergeBlock) {
         const int c = clusters[i];
         float4 lo = bmin[c], hi = bmax[c];
@@ -558,6 +582,8 @@ constexpr int kCollapseBlock = 128, kCollapseNodes = kCollapseBlock / 8;
 __global__ void __launch_bounds__(kCollapseBlock) k_collapse(CollapseArgs A, int levelIdx,
                                                              const int2 *__restrict__ items, int2 *__restrict__ next) {
     __shared__ unsigned long long alloc[kCollapseNodes];
+    cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
     // nodes and triangles placed by the levels before this one; this level's items
     int nodeBase = 1, triBase0 = 0;
     for (int l = 0; l < levelIdx; l++) {
@@ -872,14 +898,21 @@ int buildWideBVH(const float *d_verts, int n, const int *d_tri_mat, const int *d
             }
             for (int k = 0; k < kRoundsAhead; k++, r++) {
                 const int *in = clusters[r & 1];
-                k_ploc_nn<<<(st.m + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, stream>>>(in, rounds + r, bmin, bmax, nn);
-                k_ploc_count<<<(st.m + kMergeBlock - 1) / kMergeBlock, kMergeBlock, 0, stream>>>(nn, rounds + r, sums);
-                k_ploc_merge<<<(st.m + kMergeBlock - 1) / kMergeBlock, kMergeBlock, 0, stream>>>(
-                    in, rounds + r, nn, sums, child, bmin, bmax, count, clusters[(r & 1) ^ 1]);
-                k_dp_round<<<(st.m / 2 + T - 1) / T, T, 0, stream>>>(child, count, bmin, bmax, rounds + r, n, dp);
+                // at most half of the last round's clusters merged; a few blocks run over more
+                const int dpBlocks = r == 0 ? 0 : std::min((st.m / 2 + kMergeBlock - 1) / kMergeBlock, 152);
+                const int blocks = (st.m + kMergeBlock - 1) / kMergeBlock;
+                if (e == cudaSuccess)
+                    e = launchDependent(k_ploc_nn, dim3((st.m + kPlocBlock - 1) / kPlocBlock), dim3(kPlocBlock), 0, stream,
+                                        k > 0, in, rounds + r, bmin, bmax, nn);
+                if (e == cudaSuccess)
+                    e = launchDependent(k_ploc_count, dim3(dpBlocks + blocks), dim3(kMergeBlock), 0, stream, true, nn,
+                                        rounds + r, sums, dpBlocks, child, count, bmin, bmax, n, dp);
+                if (e == cudaSuccess)
+                    e = launchDependent(k_ploc_merge, dim3(blocks), dim3(kMergeBlock), 0, stream, true, in, rounds + r, nn,
+                                        sums, child, bmin, bmax, count, clusters[(r & 1) ^ 1]);
             }
             const int before = st.m;
-            e = cudaMemcpyAsync(&st, rounds + r, sizeof(st), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(&st, rounds + r, sizeof(st), cudaMemcpyDeviceToHost, stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
             if (e == cudaSuccess && st.m >= before) {
                 snprintf(err, errlen, "buildWideBVH: clustering made no progress");
@@ -891,7 +924,7 @@ int buildWideBVH(const float *d_verts, int n, const int *d_tri_mat, const int *d
             e = cudaFuncSetAttribute(k_ploc_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailSmem);
             if (e == cudaSuccess)
                 k_ploc_tail<<<1, kMergeBlock, kTailSmem, stream>>>(clusters[r & 1], rounds + r, child, bmin, bmax,
-                                                                   count, n, dp);
+                                                                   count, n, r > 0, dp);
         }
         // the wide tree, kRoundsAhead levels between two looks at what they allocated
         const int2 root = make_int2(n > 1 ? 0 : n - 1, 0);
@@ -908,11 +941,13 @@ int buildWideBVH(const float *d_verts, int n, const int *d_tri_mat, const int *d
             if (depth > 0) most = static_cast<long long>(got[depth - 1] & 0xFFFFFFFFull);
             for (int k = 0; k < kRoundsAhead && depth + k < kMaxLevels; k++) {
                 const long long blocks = (std::min<long long>(most, n) + kCollapseNodes - 1) / kCollapseNodes;
-                k_collapse<<<static_cast<int>(std::min<long long>(blocks, 152 * 16)), kCollapseBlock, 0, stream>>>(
-                    A, depth + k, items[(depth + k) & 1], items[((depth + k) & 1) ^ 1]);
+                if (e == cudaSuccess)
+                    e = launchDependent(k_collapse, dim3(static_cast<unsigned>(std::min<long long>(blocks, 152 * 16))),
+                                        dim3(kCollapseBlock), 0, stream, k > 0, A, depth + k, items[(depth + k) & 1],
+                                        items[((depth + k) & 1) ^ 1]);
                 most = std::min<long long>(8 * most, n);
             }
-            e = cudaMemcpyAsync(got, level, sizeof(got), cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(got, level, sizeof(got), cudaMemcpyDeviceToHost, stream);
             if (e == cudaSuccess && depth == 0)
                 e = cudaMemcpyAsync(&left, rounds + r + 1, sizeof(left), cudaMemcpyDeviceToHost, stream);
             if (e == cudaSuccess && depth == 0) e = cudaMemcpyAsync(hb, d_bounds, sizeof(hb), cudaMemcpyDeviceToHost, stream);

@@ -724,4 +724,22 @@ __device__ __forceinline__ void narrowType(MaterialRecord &m) {
 
 __device__ __forceinline__ float powerHeuristic(float f, float g) { return (f * f) / (f * f + g * g); }
 
+// a launch that may begin (up to its cudaGridDependencySynchronize) while the stream's last kernel
+// ends, if dependent
+template <class... Params, class... Args>
+cudaError_t launchDependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool dependent,
+                            Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 }  // namespace spgpu

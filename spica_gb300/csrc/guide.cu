@@ -914,24 +914,6 @@ int tmemKernelResidentCtas(const void *kernel, int device, int dynSmem = kGuided
     return std::max(1, std::min(std::min(byRegs, bySmem), std::min(std::min(byThreads, blkSM), byTmem)));
 }
 
-// a launch that may begin (up to its cudaGridDependencySynchronize) while the stream's last kernel
-// ends, if dependent
-template <class... Params, class... Args>
-cudaError_t launchDependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool dependent,
-                            Args... args) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = dependent ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
-
 template <class T>
 T *galloc(size_t n) {
     T *p = nullptr;
