@@ -102,6 +102,23 @@ def test_durand_non_finite_pixel(gpulib):
     np.testing.assert_array_equal(_resolve(film, gpu.FILM_DURAND, 5.0), want)
 
 
+@pytest.mark.parametrize("odd", [(-5e-7, -5e-7, -5e-7, 1.0), (0.0, 0.0, 0.0, 0.0), (1.0, 2.0, 3.0, 0.0),
+                                 (1e30, 1.0, 1.0, 1.0)])
+@pytest.mark.parametrize("contrast", [0.5, 5.0, 200.0])
+def test_durand_odd_pixels(gpulib, contrast, odd):
+    """The detail layer as a factor where the reference takes its logarithm: a negative one has
+    none, and its pixel clamps to 0 (tolerances as in test_durand_chunked_filter)."""
+    from oracle import tmo_oracle
+    from spica_gb300 import gpu
+    rng = np.random.default_rng(3)
+    film = np.concatenate([rng.lognormal(0, 2.0, (33, 47, 3)), np.full((33, 47, 1), 4.0)], -1).astype(np.float32)
+    film[rng.random((33, 47)) < 0.05, :3] = 0.0
+    film[12, 20] = odd
+    with np.errstate(all="ignore"):
+        want = tmo_oracle.durand(film, contrast)
+    np.testing.assert_allclose(_resolve(film, gpu.FILM_DURAND, contrast), want, rtol=2e-6, atol=1e-12)
+
+
 @pytest.mark.parametrize("odd", [None, (0.0, 0.0, 0.0, 0.0), (-1.0, 0.2, 0.1, 1.0), (1.0, 2.0, 3.0, 0.0),
                                  (np.inf, 1.0, 1.0, 4.0), (1.0, np.nan, 1.0, 4.0)])
 @pytest.mark.parametrize("param", [0.18, 0.5, 0.85, 1.0, 1.7])
