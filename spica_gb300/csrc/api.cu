@@ -208,7 +208,9 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_trace(const float4 *__restri
     uint32_t nodeCount = 0, triCount = 0;
     bool overflow = false;
     auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1) {
-        const float4 a = org[i], b = dir[i];
+        // rays and hits as streaming data, which leaves the caches to the tree: 16M closest hits
+        // 3.17 -> 3.14 ms
+        const float4 a = __ldcs(org + i), b = __ldcs(dir + i);
         *o = xyz(a);
         *d = xyz(b);
         *t0 = a.w;
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_trace(const float4 *__restri
     auto done = [&](int i, const TraceLane &L) {
         if (i < 0) return;
         if (ANY) {
-            outAny[i] = L.found ? 1u : 0u;
+            __stcs(outAny + i, L.found ? 1u : 0u);
             return;
         }
         float t = L.tmax, u = L.hu, v = L.hv;
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) k_trace(const float4 *__restri
             if (!(kappa < 16.0f * det)) refineHitFP64(tr, L.o, L.d, &t, &u, &v);
             prim = __float_as_int(tr.v0.w);
         }
-        reinterpret_cast<float4 *>(outHit)[i] = make_float4(L.found ? t : 0.0f, __int_as_float(prim), u, v);
+        __stcs(reinterpret_cast<float4 *>(outHit) + i, make_float4(L.found ? t : 0.0f, __int_as_float(prim), u, v));
     };
     tracePersistent<ANY, STATS, SPLIT, OWN>(nodes, tris, nNodes, nTris, n, ctl + 1, stack + threadIdx.x, kTraceBlock, &nodeCount,
                                 &triCount, &overflow, fetch, done);

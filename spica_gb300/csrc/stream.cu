@@ -27,7 +27,9 @@
 // The iterations are captured into one CUDA graph of kIterPerGraph iterations, replayed
 // until the device reports that every path of the render has ended.  The host reads the
 // done flag of the replay kReplayLag launches back, so the GPU always has work queued;
-// replays past the end find empty queues and return at once.
+// replays past the end find empty queues and return at once.  A render whose paths fit the
+// pools at once runs without the graph, one vertex depth per iteration (renderOnePass).
+// Scenes of one material class are shaded from the pool itself, without class queues.
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -151,6 +153,13 @@ struct StreamArgs {
     long long iterLimit;
 };
 
+// The path records (pool, class queues, hits, shadow queue) are written once and read once, by
+// another kernel and far apart, so they are loaded and stored as streaming data (evict first):
+// L1 and L2 keep the tree, the triangles and the materials.  Default policy against loads / both
+// as streaming: a batch of 16 box rooms 145.1 / 145.0 / 142.3 ms, the mid-scale scene at 1080p
+// with 16 samples 25.6 / 25.4 / 25.1, the material room at 333 x 217 1.31 / 1.30 / 1.28, the
+// guided room 3.17 / 3.13 / 3.12.
+
 __device__ __forceinline__ int filmIndexS(const StreamArgs &p, int pix) {
     const int y = pix / p.W, x = pix - y * p.W;
     return y * p.W + (p.W - 1 - x);   // film pixel (W-1-x, y), core/integrator.cc:88
@@ -242,9 +251,9 @@ __global__ void k_sregen(StreamArgs p) {
             spawnCameraRay(p.cam, x, y, r.a, r.b, &o, &d);
         }
         const int k = have + j;
-        p.rO[k] = make_float4(o.x, o.y, o.z, __int_as_float(pix));
-        p.rD[k] = make_float4(d.x, d.y, d.z, packMeta(0, false, render));
-        p.rB[k] = make_float4(1.0f, 1.0f, 1.0f, __int_as_float(sample));
+        __stcs(&p.rO[k], make_float4(o.x, o.y, o.z, __int_as_float(pix)));
+        __stcs(&p.rD[k], make_float4(d.x, d.y, d.z, packMeta(0, false, render)));
+        __stcs(&p.rB[k], make_float4(1.0f, 1.0f, 1.0f, __int_as_float(sample)));
         atomicAdd(&film[filmBase + fi].w, 1.0f);
     }
 }
@@ -262,13 +271,14 @@ __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
         if constexpr (SINGLE) {
             int render = 0;
             if (i >= 0) {
-                p.qH[i] = make_float4(L.tmax, __int_as_float(L.found ? L.hitSlot : -1), L.hu, L.hv);
+                __stcs(&p.qH[i], make_float4(L.tmax, __int_as_float(L.found ? L.hitSlot : -1), L.hu, L.hv));
                 if (!L.found && (BATCH || p.sv.hasEnv)) {
-                    const int meta = __float_as_int(p.rD[i].w);
+                    const int meta = __float_as_int(__ldcs(&p.rD[i]).w);
                     if (BATCH) render = metaRender(meta);
                     else if ((meta & 255) == 0 || (meta & 256)) {
-                        const float3 c = xyz(p.rB[i]) * envLe(p.sv.env, L.d);
-                        atomicAdd(&film[filmIndexS(p, __float_as_int(p.rO[i].w))], make_float4(c.x, c.y, c.z, 0.0f));
+                        const float3 c = xyz(__ldcs(&p.rB[i])) * envLe(p.sv.env, L.d);
+                        const int pix = __float_as_int(__ldcs(&p.rO[i]).w);
+                        atomicAdd(&film[filmIndexS(p, pix)], make_float4(c.x, c.y, c.z, 0.0f));
                     }
                 }
             }
@@ -278,9 +288,9 @@ __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
         int cls = -1;
         float4 o4 = make_float4(0, 0, 0, 0), d4 = o4, b4 = o4;
         if (i >= 0) {
-            o4 = p.rO[i];
-            d4 = p.rD[i];
-            b4 = p.rB[i];
+            o4 = __ldcs(&p.rO[i]);
+            d4 = __ldcs(&p.rD[i]);
+            b4 = __ldcs(&p.rB[i]);
             if (L.found) {
                 cls = shadeClass(__ldg(&p.sv.mats[__ldg(&p.sv.slotShade[L.hitSlot]).x].type));
             } else if (!BATCH && p.sv.hasEnv) {
@@ -298,18 +308,18 @@ __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
             const int k = warpAppendS(cls == c, &p.ctr[kCtrClass0 + c]);
             if (k >= 0) {
                 const int64_t row = static_cast<int64_t>(c) * p.cap + k;
-                p.qO[row] = o4;
-                p.qD[row] = d4;
-                p.qB[row] = b4;
-                p.qH[row] = make_float4(L.tmax, __int_as_float(L.hitSlot), L.hu, L.hv);
+                __stcs(&p.qO[row], o4);
+                __stcs(&p.qD[row], d4);
+                __stcs(&p.qB[row], b4);
+                __stcs(&p.qH[row], make_float4(L.tmax, __int_as_float(L.hitSlot), L.hu, L.hv));
             }
         }
     };
     if constexpr (BATCH) {
         // each render's rays start at its own tree's root
         auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1, uint32_t *root) {
-            const float4 d4 = p.rD[i];
-            *o = xyz(p.rO[i]);
+            const float4 d4 = __ldcs(&p.rD[i]);
+            *o = xyz(__ldcs(&p.rO[i]));
             *d = xyz(d4);
             *t0 = 0.0f;
             *t1 = kInfT;
@@ -320,8 +330,8 @@ __device__ __forceinline__ void extendQueue(const StreamArgs &p, uint2 *stack) {
                                       done);
     } else {
         auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1) {
-            *o = xyz(p.rO[i]);
-            *d = xyz(p.rD[i]);
+            *o = xyz(__ldcs(&p.rO[i]));
+            *d = xyz(__ldcs(&p.rD[i]));
             *t0 = 0.0f;
             *t1 = kInfT;
         };
@@ -346,9 +356,9 @@ __global__ void __launch_bounds__(kTraceBlock, kTraceMinBlocks) k_sextend(Stream
 // shading append together
 __device__ __forceinline__ void appendShadow(const StreamArgs &p, float4 so, float4 sd, float4 sl) {
     const int k = warpAppendS(true, &p.ctr[kCtrShadow]);
-    p.shO[k] = so;
-    p.shD[k] = sd;
-    p.shL[k] = sl;
+    __stcs(&p.shO[k], so);
+    __stcs(&p.shD[k], sd);
+    __stcs(&p.shL[k], sl);
 }
 
 // a shaded hit's emission (at film pixel filmIdx) and continuation (back into the pool);
@@ -361,9 +371,9 @@ __device__ __forceinline__ void emitShadeResultS(const StreamArgs &p, const Shad
     if constexpr (BATCH) countEnded(p, live && !R.cont, metaRender(meta));
     const int k = warpAppendS(R.cont && !p.direct, p.cont);
     if (k >= 0) {
-        p.nO[k] = make_float4(R.cO.x, R.cO.y, R.cO.z, __int_as_float(pix));
-        p.nD[k] = make_float4(R.cD.x, R.cD.y, R.cD.z, packMeta((meta & 255) + 1, R.spec, metaRender(meta)));
-        p.nB[k] = make_float4(R.beta.x, R.beta.y, R.beta.z, __int_as_float(sample));
+        __stcs(&p.nO[k], make_float4(R.cO.x, R.cO.y, R.cO.z, __int_as_float(pix)));
+        __stcs(&p.nD[k], make_float4(R.cD.x, R.cD.y, R.cD.z, packMeta((meta & 255) + 1, R.spec, metaRender(meta))));
+        __stcs(&p.nB[k], make_float4(R.beta.x, R.beta.y, R.beta.z, __int_as_float(sample)));
     }
 }
 
@@ -429,11 +439,11 @@ __global__ void __launch_bounds__(kShadeBlockS, shadeMinBlocks(CLS)) k_sshade(St
         bool live = false;
         float4 h4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (j < n) {
-            h4 = rows.h[j];
+            h4 = __ldcs(rows.h + j);
             live = p.singleClass < 0 || __float_as_int(h4.y) >= 0;   // a class queue holds hits only
         }
         if (live) {
-            const float4 o4 = rows.o[j], d4 = rows.d[j], b4 = rows.b[j];
+            const float4 o4 = __ldcs(rows.o + j), d4 = __ldcs(rows.d + j), b4 = __ldcs(rows.b + j);
             pix = __float_as_int(o4.w);
             meta = __float_as_int(d4.w);
             sample = __float_as_int(b4.w);
@@ -491,10 +501,10 @@ __global__ void __launch_bounds__(kGTile, kGuidedMinBlocks) k_sshade_guided(Stre
         float4 o4 = make_float4(0, 0, 0, 0), d4 = make_float4(0, 0, 1, 0), b4 = o4;
         float4 h4 = make_float4(0.0f, __int_as_float(-1), 0.0f, 0.0f);
         if (j < n) {
-            o4 = rows.o[j];
-            d4 = rows.d[j];
-            b4 = rows.b[j];
-            h4 = rows.h[j];
+            o4 = __ldcs(rows.o + j);
+            d4 = __ldcs(rows.d + j);
+            b4 = __ldcs(rows.b + j);
+            h4 = __ldcs(rows.h + j);
         }
         const bool live = __float_as_int(h4.y) >= 0;
         float3 ps = mk(0, 0, 0), nn = mk(0, 0, 1);
@@ -552,14 +562,14 @@ __device__ __forceinline__ void shadowQueue(const StreamArgs &p, int *ctr, uint2
     uint32_t nodeCount = 0, triCount = 0;
     auto done = [&](int i, const TraceLane &L) {
         if (i >= 0 && !L.found) {
-            const float3 c = xyz(p.shL[i]);
-            atomicAdd(&film[__float_as_int(p.shO[i].w)], make_float4(c.x, c.y, c.z, 0.0f));
+            const float3 c = xyz(__ldcs(&p.shL[i]));
+            atomicAdd(&film[__float_as_int(__ldcs(&p.shO[i]).w)], make_float4(c.x, c.y, c.z, 0.0f));
         }
     };
     if constexpr (BATCH) {
         auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1, uint32_t *root) {
-            const float4 d4 = p.shD[i];
-            *o = xyz(p.shO[i]);
+            const float4 d4 = __ldcs(&p.shD[i]);
+            *o = xyz(__ldcs(&p.shO[i]));
             *d = xyz(d4);
             *t0 = 0.0f;
             *t1 = d4.w;
@@ -569,8 +579,8 @@ __device__ __forceinline__ void shadowQueue(const StreamArgs &p, int *ctr, uint2
                                      stack + threadIdx.x, kTraceBlock, &nodeCount, &triCount, &overflow, fetch, done);
     } else {
         auto fetch = [&](int i, float3 *o, float3 *d, float *t0, float *t1) {
-            const float4 d4 = p.shD[i];
-            *o = xyz(p.shO[i]);
+            const float4 d4 = __ldcs(&p.shD[i]);
+            *o = xyz(__ldcs(&p.shO[i]));
             *d = xyz(d4);
             *t0 = 0.0f;
             *t1 = d4.w;
@@ -1205,8 +1215,8 @@ long long oneLanePaths(const StreamArgs &a) {
 // iteration's launch, and the classes that the scene has no material of are not launched: two
 // kernels for an iteration of a one-class scene instead of seven.  Bound by the launches' own
 // latency at the small end.  Against the refilling loop's replays: box room, 64 x 64, 16
-// samples (host film) 1.00 -> 0.43 ms; material room, 333 x 217, 24 samples 1.82 -> 1.32;
-// guided room, 640 x 360, 8 samples 4.04 -> 3.32.
+// samples (host film) 1.00 -> 0.43 ms (0.26 with the context's kept host film); material room,
+// 333 x 217, 24 samples 1.82 -> 1.32; guided room, 640 x 360, 8 samples 4.04 -> 3.23.
 int renderOnePass(Ctx &C, const float *camera, int W, int H, int spp, int sampleOffset, int maxDepth, uint32_t seed,
                   int integrator, float4 *film, unsigned long long *statsOut, float *msOut, cudaStream_t stream,
                   const GuideView *gv) {
