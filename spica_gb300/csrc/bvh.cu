@@ -195,7 +195,7 @@ __global__ void k_leaf_bounds(const float *__restrict__ verts, const uint32_t *_
 struct RoundState {
     int m, top;
 };
-constexpr int kRoundsAhead = 4;
+constexpr int kRoundsAhead = 8;   // 4 / 6 / 8: 2M triangles 3.18 / 3.12 / 3.08 ms, 16k 0.98 / 0.95 / 0.97
 constexpr int kMaxRounds = 1024;
 constexpr int kTailClusters = 2048;
 constexpr int kMergeBlock = 1024;
