@@ -27,7 +27,7 @@ guided  the guiding room at 640 x 360: 8 collection passes of 2 spp with 32 Adam
         evaluation of 65,536 inputs (k_guide_forward)
 train   the guiding room at 1280 x 720: 8 collection passes of 2 spp, 16 + 64 Adam steps
         of 16,384 samples (host-timed), then 20 steps inside the NVTX range "profiled"
-        (k_gather, k_guide_train, k_grad_sum, k_guide_pack)
+        (k_guide_train, k_step_update)
 build   the device BVH build of the mid-scale scene, or of the microbench sphere with
         --levels (Morton keys, clustering rounds, SAH programme, collapse)
 film    a rendered box room at W x H resolved by every film format (RGBE, gamma,
