@@ -30,7 +30,7 @@
 // A build was bound by what surrounds its kernels: some 75 clustering rounds of eight launches
 // and a host round trip each, 30 allocations, and one thread per wide node in the collapse.  With
 // rounds that run ahead of the host, the last rounds in one block, one scratch allocation and
-// eight threads per wide node, 2.03M triangles take 11.4 -> 3.2 ms, 256 triangles 1.96 -> 0.28.
+// eight threads per wide node, 2.03M triangles take 11.4 -> 2.9 ms, 256 triangles 1.96 -> 0.28.
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
@@ -147,7 +147,7 @@ __device__ __forceinline__ float areaOf(float4 lo, float4 hi) {
 
 // ---------------------------------------------------------------- clustering
 constexpr int kPlocRadius = 32;   // neighbours searched on each side, in code order
-constexpr int kPlocBlock = 256;
+constexpr int kPlocBlock = 256;   // clusters of a block of k_ploc_nn
 
 // leaves: node n-1+j is the j-th triangle in code order
 // SAH weights of the wide tree: a wide-node visit, a triangle test.  Equal weights were
@@ -202,44 +202,62 @@ constexpr int kMergeBlock = 1024;
 
 // nearest neighbour of each cluster: least surface area of the merged box among the
 // clusters within kPlocRadius positions (ties: the lower position); the window's boxes
-// are staged in shared memory
-__global__ void __launch_bounds__(kPlocBlock) k_ploc_nn(const int *__restrict__ clusters,
-                                                        const RoundState *__restrict__ round,
-                                                        const float4 *__restrict__ bmin,
-                                                        const float4 *__restrict__ bmax, int *nn) {
-    __shared__ float4 slo[kPlocBlock + 2 * kPlocRadius], shi[kPlocBlock + 2 * kPlocRadius];
+// are staged in shared memory, and reading them from there is what bounds this.  So a thread
+// takes two neighbouring clusters, whose windows share all but their ends, and each box read
+// serves both; even and odd positions have their own arrays, so that the threads' reads, two
+// positions apart, fall on different banks.  Beyond the first and last cluster the arrays hold
+// boxes of infinite area.  2M triangles 3.05 -> 2.91 ms (2.95 / 3.00 / 3.02 unrolled by 11 / 3 /
+// not at all), 256k 1.54 -> 1.49; blocks of 512 clusters 3.02.
+__global__ void __launch_bounds__(kPlocBlock / 2) k_ploc_nn(const int *__restrict__ clusters,
+                                                            const RoundState *__restrict__ round,
+                                                            const float4 *__restrict__ bmin,
+                                                            const float4 *__restrict__ bmax, int *nn) {
+    constexpr int kSpan = kPlocBlock + 2 * kPlocRadius, kHalf = kPlocRadius / 2;
+    static_assert(kPlocRadius % 2 == 0 && kPlocBlock % 2 == 0, "a thread's first cluster is at an even position");
+    __shared__ float4 slo[2][kSpan / 2], shi[2][kSpan / 2];
     cudaGridDependencySynchronize();
     cudaTriggerProgrammaticLaunchCompletion();
     const int m = round->m;
     if (m <= kTailClusters || static_cast<int>(blockIdx.x) * kPlocBlock >= m) return;
     const int base = blockIdx.x * kPlocBlock - kPlocRadius;
-    for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock) {
+    for (int k = threadIdx.x; k < kSpan; k += kPlocBlock / 2) {
         const int p = base + k;
+        float4 lo = make_float4(-1e30f, -1e30f, -1e30f, 0.0f), hi = make_float4(1e30f, 1e30f, 1e30f, 0.0f);
         if (p >= 0 && p < m) {
             const int c = clusters[p];
-            slo[k] = bmin[c];
-            shi[k] = bmax[c];
+            lo = bmin[c];
+            hi = bmax[c];
         }
+        slo[k & 1][k >> 1] = lo;
+        shi[k & 1][k >> 1] = hi;
     }
     __syncthreads();
-    const int i = blockIdx.x * kPlocBlock + threadIdx.x;
+    const int i = blockIdx.x * kPlocBlock + 2 * static_cast<int>(threadIdx.x);   // and i + 1
     if (i >= m) return;
-    const int li = threadIdx.x + kPlocRadius;
-    const float4 lo = slo[li], hi = shi[li];
-    float best = 3.0e38f;
-    int bestJ = -1;
-    for (int d = -kPlocRadius; d <= kPlocRadius; d++) {
-        const int j = i + d;
-        if (d == 0 || j < 0 || j >= m) continue;
-        const float4 a = slo[li + d], b = shi[li + d];
+    const int own = threadIdx.x + kHalf;
+    const float4 lo0 = slo[0][own], hi0 = shi[0][own], lo1 = slo[1][own], hi1 = shi[1][own];
+    float best0 = 3.0e38f, best1 = 3.0e38f;
+    int at0 = -1, at1 = -1;
+    auto closer = [](const float4 &lo, const float4 &hi, const float4 &a, const float4 &b, int j, float *best, int *at) {
         const float area = areaOf(make_float4(fminf(lo.x, a.x), fminf(lo.y, a.y), fminf(lo.z, a.z), 0.0f),
                                   make_float4(fmaxf(hi.x, b.x), fmaxf(hi.y, b.y), fmaxf(hi.z, b.z), 0.0f));
-        if (area < best) {
-            best = area;
-            bestJ = j;
+        if (area < *best) {
+            *best = area;
+            *at = j;
         }
+    };
+#pragma unroll
+    for (int e = -kHalf; e <= kHalf; e++) {   // positions i + 2 e and i + 2 e + 1
+        const int j = i + 2 * e;
+        const float4 a0 = slo[0][own + e], b0 = shi[0][own + e];
+        if (e != 0) closer(lo0, hi0, a0, b0, j, &best0, &at0);
+        if (e != -kHalf) closer(lo1, hi1, a0, b0, j, &best1, &at1);
+        const float4 a1 = slo[1][own + e], b1 = shi[1][own + e];
+        if (e != kHalf) closer(lo0, hi0, a1, b1, j + 1, &best0, &at0);
+        if (e != 0) closer(lo1, hi1, a1, b1, j + 1, &best1, &at1);
     }
-    nn[i] = bestJ;
+    nn[i] = at0;
+    if (i + 1 < m) nn[i + 1] = at1;
 }
 
 // A cluster leads a merge when it and its neighbour chose each other and it comes first; it
@@ -902,8 +920,8 @@ int buildWideBVH(const float *d_verts, int n, const int *d_tri_mat, const int *d
                 const int dpBlocks = r == 0 ? 0 : std::min((st.m / 2 + kMergeBlock - 1) / kMergeBlock, 152);
                 const int blocks = (st.m + kMergeBlock - 1) / kMergeBlock;
                 if (e == cudaSuccess)
-                    e = launchDependent(k_ploc_nn, dim3((st.m + kPlocBlock - 1) / kPlocBlock), dim3(kPlocBlock), 0, stream,
-                                        k > 0, in, rounds + r, bmin, bmax, nn);
+                    e = launchDependent(k_ploc_nn, dim3((st.m + kPlocBlock - 1) / kPlocBlock), dim3(kPlocBlock / 2), 0,
+                                        stream, k > 0, in, rounds + r, bmin, bmax, nn);
                 if (e == cudaSuccess)
                     e = launchDependent(k_ploc_count, dim3(dpBlocks + blocks), dim3(kMergeBlock), 0, stream, true, nn,
                                         rounds + r, sums, dpBlocks, child, count, bmin, bmax, n, dp);
