@@ -158,7 +158,9 @@ struct StreamArgs {
 // L1 and L2 keep the tree, the triangles and the materials.  Default policy against loads / both
 // as streaming: a batch of 16 box rooms 145.1 / 145.0 / 142.3 ms, the mid-scale scene at 1080p
 // with 16 samples 25.6 / 25.4 / 25.1, the material room at 333 x 217 1.31 / 1.30 / 1.28, the
-// guided room 3.17 / 3.13 / 3.12.
+// guided room 3.17 / 3.13 / 3.12.  (Rays that the end of a traversal reads again come from DRAM
+// again, 262 instead of 202 MB an average extend launch of that frame; keeping those in the
+// caches costs the tree 0.6-1 %.)
 
 __device__ __forceinline__ int filmIndexS(const StreamArgs &p, int pix) {
     const int y = pix / p.W, x = pix - y * p.W;
